@@ -177,6 +177,14 @@ int td3_m2l_tensor(const i64* row_start, const int* entry_row, const i64* partne
                    const float2* hat, int order, const double* coeff, double unit,
                    double* local_re, double* local_im, i64* status, cudaStream_t s);
 
+// The Cartesian M2L of orders up to 16 from the moments themselves (cart_m2l.cu): arguments
+// as td3_cart_m2l_mixed; FP64 without `mixed` (the half-widths are then not read).
+int td3_cart_m2l_unpacked(const i64* row_start, const i64* partners, i64 n_dst,
+                          const double* dst_center, const double* dst_half,
+                          const double* src_center, const double* src_half,
+                          const double* moments, int order, double softening, bool mixed,
+                          double* local, cudaStream_t s);
+
 // Stable LSD radix sort of (key, value) pairs by the low `bits` bits of the key
 // (scan.cu).  Keys and values are ping-ponged between the in and alt buffers; the
 // sorted result is returned in *keys_out / *vals_out (one of the two buffers).

@@ -1258,11 +1258,17 @@ class FlatQuadtree:
         if moments is None:
             moments = self._cartesian_moments()
         local = torch.zeros((dst.node_count, n_coef), dtype=torch.float64, device=self.device)
-        if n_m2l and self.precision == "mixed" and self.order <= 16:
-            _lib.call("td3_cart_m2l_mixed", rows.data_ptr(), partners.data_ptr(), dst.node_count,
+        if n_m2l and self.order <= 16:
+            width = _lib.lib().td3_cart_record_bytes(self.order, self._mixed)
+            records = torch.empty((self.node_count, width), dtype=torch.uint8,
+                                  device=self.device)
+            _lib.call("td3_pack_cart_sources", self.node_count, self.order, moments.data_ptr(),
+                      self.node_half.data_ptr(), self._mixed, records.data_ptr(), stream)
+            _lib.call("td3_cart_m2l_rows", rows.data_ptr(), partners.data_ptr(), dst.node_count,
                       dst.node_center.data_ptr(), dst.node_half.data_ptr(),
                       self.node_center.data_ptr(), self.node_half.data_ptr(),
-                      moments.data_ptr(), self.order, float(softening), local.data_ptr(), stream)
+                      records.data_ptr(), self.order, float(softening), self._mixed,
+                      local.data_ptr(), stream)
         elif n_m2l:
             _lib.call("td3_cart_m2l", rows.data_ptr(), partners.data_ptr(), dst.node_count,
                       dst.node_center.data_ptr(), self.node_center.data_ptr(),
