@@ -76,7 +76,7 @@ k_m2l_cart(const i64* __restrict__ row_start, const i64* __restrict__ partners, 
     }
 }
 
-// L2L of one level: a block per (node, child), thread b: T_b(child) += sum_g C(g, b) T_g
+// L2L of one level (orders above 16): a block per (node, child), thread b: T_b(child) += sum_g C(g, b) T_g
 // s^(g-b) over the rows of b (g, d = g - b, coef).  The monomials s^d are built once per
 // block into shared memory, column d_y by thread d_y as the reference's mono recurrence
 // builds them (d_y factors of s_y, then s_x one at a time).
@@ -105,6 +105,112 @@ __global__ void k_l2l_cart(i64 lo, int order, int n_coef, const double* __restri
             acc += l2l_coef[r] * local[node * n_coef + l2l_g[r]] * shift_mono[l2l_d[r]];
         local[ch * n_coef + b] += acc;
     }
+}
+
+// The L2L of orders up to 16 (template order P): the shift by (s_x, s_y) as two passes of
+// one-dimensional Taylor shifts (C(p + 3, 3) multiply-adds each against C(p + 4, 4) for the
+// table rows: 910 against 1820 at p = 12), a thread per (child, row) with its row in
+// registers.  A parent's coefficients are read once for its four children, whose rows are one
+// contiguous run of the locals.  Measured (p = 12, all levels; a block per child over the
+// table rows before): 2.9 -> 0.58 ms for 1M clustered particles (the locals alone move 0.1 ms),
+// 0.36 -> 0.07 ms for 100k uniform ones.
+template <int P>
+struct CartL2L {
+    static constexpr int W = P + 1, TILE = W * W;
+    static constexpr int THREADS = P == 4 ? 32 : P == 16 ? 96 : 64;  // per parent, >= 4 W
+    static constexpr int NODES = P == 4 ? 4 : 2;                     // parents per block, each step
+};
+
+// t_b <- sum_(g >= b) C(g, b) s^(g - b) t_g
+template <int W>
+__device__ __forceinline__ void taylor_shift(double (&t)[W], double s) {
+#pragma unroll
+    for (int i = 0; i < W - 1; ++i)
+#pragma unroll
+        for (int b = W - 2; b >= i; --b) t[b] += s * t[b + 1];
+}
+
+template <int P>
+__global__ void __launch_bounds__(CartL2L<P>::THREADS* CartL2L<P>::NODES)
+k_l2l_cart_rows(i64 lo, i64 hi, int span, int order, const double* __restrict__ center,
+                const i64* __restrict__ child, double* local) {
+    typedef CartL2L<P> L;
+    constexpr int W = L::W, TILE = L::TILE;
+    __shared__ double own[L::NODES][TILE], out[L::NODES][4][TILE];  // squares [y][x]
+    __shared__ short place[W * (W + 1) / 2];  // of a coefficient in a square
+    __shared__ int list[32], count;
+    const int n_coef = (order + 1) * (order + 2) / 2;
+    const int slot = threadIdx.x / L::THREADS, me = threadIdx.x % L::THREADS;
+    for (int i = threadIdx.x; i < TILE; i += blockDim.x) {
+        const int x = i % W, y = i / W;
+        if (x + y <= order) place[(x + y) * (x + y + 1) / 2 + y] = (short)i;
+    }
+    const int k = me / W, r = me % W;  // child and row
+    td3_chain_wait();
+    td3_chain_release();
+    const i64 first = lo + (i64)blockIdx.x * span;
+    if (threadIdx.x < 32) {  // the parents among the block's cells
+        const i64 node = first + threadIdx.x;
+        const bool take = (int)threadIdx.x < span && node < hi && child[node] >= 0;
+        const unsigned m = __ballot_sync(0xffffffffu, take);
+        if (take) list[__popc(m & ((1u << threadIdx.x) - 1u))] = threadIdx.x;
+        if (threadIdx.x == 0) count = __popc(m);
+    }
+    __syncthreads();
+    for (int base = 0; base < count; base += L::NODES) {
+        const bool live = base + slot < count;
+        const i64 node = first + list[live ? base + slot : base];
+        const i64 kids = child[node];
+        if (live) {
+            for (int c = me; c < n_coef; c += L::THREADS)
+                own[slot][place[c]] = local[node * n_coef + c];
+        }
+        __syncthreads();
+        const bool work = live && k < 4 && r <= order;
+        double t[W];
+        if (work) {  // row (., r) along x
+            const double s = center[2 * (kids + k)] - center[2 * node];
+#pragma unroll
+            for (int x = 0; x < W; ++x) t[x] = x + r <= order ? own[slot][r * W + x] : 0.0;
+            taylor_shift<W>(t, s);
+#pragma unroll
+            for (int x = 0; x < W; ++x) out[slot][k][r * W + x] = t[x];
+        }
+        __syncthreads();
+        if (work) {  // row (r, .) along y
+            const double s = center[2 * (kids + k) + 1] - center[2 * node + 1];
+#pragma unroll
+            for (int y = 0; y < W; ++y) t[y] = y + r <= order ? out[slot][k][y * W + r] : 0.0;
+            taylor_shift<W>(t, s);
+#pragma unroll
+            for (int y = 0; y < W; ++y) out[slot][k][y * W + r] = t[y];
+        }
+        __syncthreads();
+        if (live) {
+            double* to = local + kids * n_coef;
+            for (int c = me; c < n_coef; c += L::THREADS) {
+#pragma unroll
+                for (int kid = 0; kid < 4; ++kid) to[kid * n_coef + c] += out[slot][kid][place[c]];
+            }
+        }
+        __syncthreads();
+    }
+}
+
+template <int P>
+int launch_l2l_rows(const i64* levels, i64 n_levels, int order, const double* center,
+                    const i64* child, double* local, cudaStream_t s) {
+    for (i64 level = 0; level + 1 < n_levels; ++level) {
+        const i64 lo = levels[level], hi = levels[level + 1];
+        if (hi <= lo) continue;
+        // consecutive cells a block picks its parents from: a few blocks per SM, 32 at most
+        const i64 pick = (hi - lo) / (148 * 8);
+        const int span = pick < CartL2L<P>::NODES ? CartL2L<P>::NODES : pick > 32 ? 32 : (int)pick;
+        TD3_TRY(td3_launch_chained(k_l2l_cart_rows<P>, td3_blocks(hi - lo, span),
+                                   CartL2L<P>::THREADS * CartL2L<P>::NODES, 0, s, lo, hi, span,
+                                   order, center, child, local));
+    }
+    return TD3_OK;
 }
 
 }  // namespace
@@ -141,6 +247,10 @@ extern "C" int td3_cart_downward(const int64_t* levels, int64_t n_levels, const 
                                  void* stream) {
     if (n_levels < 1 || order < 0 || order > TD3_MAX_ORDER) return TD3_EINVAL;
     cudaStream_t s = td3_stream(stream);
+    if (order <= 4) return launch_l2l_rows<4>(levels, n_levels, order, node_center, node_child, local, s);
+    if (order <= 8) return launch_l2l_rows<8>(levels, n_levels, order, node_center, node_child, local, s);
+    if (order <= 12) return launch_l2l_rows<12>(levels, n_levels, order, node_center, node_child, local, s);
+    if (order <= 16) return launch_l2l_rows<16>(levels, n_levels, order, node_center, node_child, local, s);
     int n_coef = (order + 1) * (order + 2) / 2;
     unsigned threads = (unsigned)((n_coef + 31) / 32 * 32);
     if (threads > 256) threads = 256;

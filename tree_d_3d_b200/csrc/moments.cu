@@ -455,7 +455,7 @@ int launch_log_moments(const int64_t* levels, int64_t n_levels, int order, const
     return TD3_OK;
 }
 
-// Cartesian moments with a block per node and thread g per coefficient.  The monomials
+// Cartesian moments (orders above 16) with a block per node and thread g per coefficient.  The monomials
 // u^(a,b) a particle (or a child's shift) needs are built once into shared memory, column
 // b by thread b as the reference's mono recurrence builds them (b factors of u_y, then
 // u_x one at a time; for a particle the first factor is its charge), and each
@@ -550,6 +550,253 @@ k_cart_moments_block(i64 lo, int order, int n_coef, const double* __restrict__ s
     }
 }
 
+// The Cartesian moments of orders up to 16 (template order P): every leaf in one launch, with
+// a lane per leaf and a warp per power of y (the sums in registers, the leaves' rows of
+// coefficients to global memory coalesced through shared memory), then the inner nodes level
+// by level.  Each coefficient adds the terms of k_cart_moments_block in its order with its
+// roundings, so the moments are the same bits.
+constexpr int CART_BATCH = 32;     // leaves in flight per block, a lane each
+constexpr int CART_SPAN = 128;     // consecutive nodes a block picks its leaves from
+constexpr int CART_STRIDE = 33;    // doubles between the coefficients of a tile
+
+// The nodes of [first, last) that are leaves (or not), in order, into list; returns their
+// number.  One warp's lanes; CART_SPAN nodes at most.
+__device__ int cart_pick(i64 first, i64 last, bool leaves, const i64* __restrict__ child,
+                         int* list) {
+    int n = 0;
+    const int lane = threadIdx.x & 31;
+    for (i64 base = first; base < last; base += 32) {
+        const i64 node = base + lane;
+        const bool take = node < last && (child[node] < 0) == leaves;
+        const unsigned m = __ballot_sync(0xffffffffu, take);
+        if (take) list[n + __popc(m & ((1u << lane) - 1u))] = (int)(node - first);
+        n += __popc(m);
+    }
+    return n;
+}
+
+// The moments of a batch's nodes from a tile, a warp per node.
+__device__ __forceinline__ void cart_store(const double* tile, i64 first, const int* list,
+                                           int n_here, int n_coef, double* moments) {
+    const int lane = threadIdx.x & 31;
+    for (int j = threadIdx.x >> 5; j < n_here; j += blockDim.x >> 5) {
+        double* to = moments + (first + list[j]) * n_coef;
+        for (int c = lane; c < n_coef; c += 32) to[c] = tile[c * CART_STRIDE + j];
+    }
+}
+
+// The leaves among all nodes: warp g_y sums the coefficients (., g_y) of the batch's leaves
+// over their particles, as k_cart_moments_block.
+template <int P>
+__global__ void __launch_bounds__(32 * (P + 1))
+k_cart_leaves(i64 n_nodes, int span, int order, const double* __restrict__ spos,
+              const double* __restrict__ scharge, i64 n_particles,
+              const double* __restrict__ center, const i64* __restrict__ start,
+              const i64* __restrict__ end, const i64* __restrict__ child, double* moments,
+              const double* __restrict__ sdip) {
+    constexpr int W = P + 1;
+    extern __shared__ double tile[];  // [coefficient][lane]
+    __shared__ int list[CART_SPAN];
+    __shared__ int count;
+    td3_chain_wait();
+    td3_chain_release();
+    const int lane = threadIdx.x & 31, gy = threadIdx.x >> 5;
+    const int n_coef = (order + 1) * (order + 2) / 2;
+    const i64 first = (i64)blockIdx.x * span;
+    if (gy == 0) {
+        const int n = cart_pick(first, first + span < n_nodes ? first + span : n_nodes, true, child, list);
+        if (lane == 0) count = n;
+    }
+    __syncthreads();
+    for (int base = 0; base < count; base += CART_BATCH) {
+        const int n_here = count - base < CART_BATCH ? count - base : CART_BATCH;
+        if (lane < n_here && gy <= order) {
+            const i64 node = first + list[base + lane];
+            const double xmid = center[2 * node], ymid = center[2 * node + 1];
+            double acc[W];
+#pragma unroll
+            for (int k = 0; k < W; ++k) acc[k] = 0.0;
+            for (i64 k = start[node]; k < end[node]; ++k) {
+                const double ux = spos[k] - xmid, uy = spos[n_particles + k] - ymid;
+                double v = scharge[k];
+                for (int t = 0; t < gy; ++t) v = v * uy;
+                if (!sdip) {
+#pragma unroll
+                    for (int gx = 0; gx < W; ++gx) {
+                        acc[gx] += v;
+                        v = v * ux;
+                    }
+                    continue;
+                }
+                // w: the powers (., g_y) of u alone, z: (., g_y - 1); a point dipole p = -e
+                // adds p . grad (r - c)^g
+                const double ex = sdip[k], ey = sdip[n_particles + k];
+                double w = 1.0, z = 1.0;
+                for (int t = 0; t < gy; ++t) {
+                    z = w;
+                    w = w * uy;
+                }
+                double before = 0.0;
+#pragma unroll
+                for (int gx = 0; gx < W; ++gx) {
+                    acc[gx] += v;
+                    if (gx > 0) acc[gx] -= ex * gx * before;
+                    if (gy > 0) acc[gx] -= ey * gy * z;
+                    before = w;
+                    v = v * ux;
+                    w = w * ux;
+                    z = z * ux;
+                }
+            }
+#pragma unroll
+            for (int gx = 0; gx < W; ++gx)
+                if (gx + gy <= order) tile[cart_index(gx, gy) * CART_STRIDE + lane] = acc[gx];
+        }
+        __syncthreads();
+        cart_store(tile, first, list + base, n_here, n_coef, moments);
+        __syncthreads();
+    }
+}
+
+// M2M of the inner nodes of a level with a thread per coefficient, the coefficients with the
+// most terms first (the threads of a warp then have about as many).  The children's
+// coefficients (one contiguous run) and the powers of their shifts are put into shared memory
+// as squares [x][y] for all four at once.  The terms (b_x, b_y) of a coefficient are one run
+// without branches, four steps in flight: near the root nothing but the chain of additions in
+// the reference's order, up to 4 x 49 at p = 12, is left of a level's time.
+//
+// Measured (p = 12, all launches; a table look-up and two reads of a block's shared memory per
+// term before): 4.0 -> 2.3 ms for 1M clustered particles, 0.52 -> 0.27 ms for 100k uniform
+// ones.  Bound by the scattered shared-memory reads at the large levels.  A lane per node
+// (no conflicts) takes 0.56 ms for the 100k: 33 us a level, however few its nodes.
+template <int P>
+struct CartM2M {
+    static constexpr int W = P + 1, COEFS = W * (P + 2) / 2, TILE = W * W;
+    static constexpr int THREADS = P == 4 ? 16 : (COEFS + 31) / 32 * 32;  // per node
+    static constexpr int NODES = P == 4 ? 8 : P == 8 ? 3 : 2;             // per block, each step
+    unsigned char x[COEFS], y[COEFS];  // the threads' coefficients
+};
+
+template <int P>
+__global__ void __launch_bounds__(CartM2M<P>::THREADS* CartM2M<P>::NODES)
+k_cart_m2m(i64 lo, i64 hi, int span, int order, const CartM2M<P> T,
+           const double* __restrict__ center, const i64* __restrict__ start,
+           const i64* __restrict__ end, const i64* __restrict__ child, double* moments) {
+    typedef CartM2M<P> M;
+    constexpr int W = M::W, TILE = M::TILE;
+    __shared__ double kids_m[M::NODES][4][TILE], powers[M::NODES][4][TILE];
+    __shared__ double binom[TILE];     // C(n, k) at n W + k
+    __shared__ short place[M::COEFS];  // of a coefficient in a square
+    __shared__ int list[32], count;
+    __shared__ bool filled[M::NODES][4];
+    const int n_coef = (order + 1) * (order + 2) / 2;
+    const int slot = threadIdx.x / M::THREADS, me = threadIdx.x % M::THREADS;
+    const int gx = me < n_coef ? T.x[me] : 0, gy = me < n_coef ? T.y[me] : 0;
+    if (me < n_coef) place[cart_index(gx, gy)] = (short)(gx * W + gy);
+    for (int i = threadIdx.x; i < TILE; i += blockDim.x) {
+        const int n = i / W, k = i % W;
+        int c = 1;
+        for (int j = 0; j < k; ++j) c = c * (n - j) / (j + 1);  // whole at each step
+        binom[i] = k <= n ? c : 0;
+    }
+    td3_chain_wait();
+    td3_chain_release();
+    const i64 first = lo + (i64)blockIdx.x * span;
+    if (threadIdx.x < 32) {
+        const int n = cart_pick(first, first + span < hi ? first + span : hi, false, child, list);
+        if (threadIdx.x == 0) count = n;
+    }
+    __syncthreads();
+    for (int base = 0; base < count; base += M::NODES) {
+        const bool live = base + slot < count;
+        const i64 node = first + list[live ? base + slot : base];
+        const i64 kids = child[node];
+        if (live) {
+            if (me < 4) filled[slot][me] = end[kids + me] != start[kids + me];
+            for (int c = me; c < n_coef; c += M::THREADS)
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    kids_m[slot][k][place[c]] = moments[(kids + k) * n_coef + c];
+            for (int i = me; i < 4 * (order + 1); i += M::THREADS) {
+                const int k = i & 3, dy = i >> 2;
+                const double ux = center[2 * (kids + k)] - center[2 * node];
+                const double uy = center[2 * (kids + k) + 1] - center[2 * node + 1];
+                double v = 1.0;
+                for (int t = 0; t < dy; ++t) v = v * uy;
+                for (int dx = 0; dx + dy <= order; ++dx) {
+                    powers[slot][k][dx * W + dy] = v;
+                    v = v * ux;
+                }
+            }
+        }
+        __syncthreads();
+        if (live && me < n_coef) {
+            const int terms = (gx + 1) * (gy + 1);
+            const double* cy = binom + gy * W;
+            double acc = 0.0;
+            for (int k = 0; k < 4; ++k) {
+                if (!filled[slot][k]) continue;
+                const double *m = kids_m[slot][k], *u = powers[slot][k] + gx * W + gy;
+                const double* cx = binom + gx * W;
+                int by = 0;
+#pragma unroll 4
+                for (int t = 0; t < terms; ++t) {
+                    // both binomials are whole numbers: their product is exact
+                    acc += *cx * cy[by] * m[by] * u[-by];
+                    const bool next = by == gy;
+                    by = next ? 0 : by + 1;
+                    cx += next ? 1 : 0;
+                    m += next ? W : 0;
+                    u -= next ? W : 0;
+                }
+            }
+            moments[node * n_coef + cart_index(gx, gy)] = acc;
+        }
+        __syncthreads();
+    }
+}
+
+// Leaves' nodes a block picks from: few, so that small trees still fill the GPU.
+int cart_span(i64 nodes) { return nodes <= 32 * 2 * 148 ? 32 : CART_SPAN; }
+
+template <int P>
+int launch_cart_lanes(const int64_t* levels, int64_t n_levels, int order, const double* spos,
+                      const double* scharge, int64_t n, const double* center, const i64* start,
+                      const i64* end, const i64* child, double* moments, const double* sdip,
+                      cudaStream_t s) {
+    const i64 count = levels[n_levels];
+    if (count <= 0) return TD3_OK;
+    const int n_coef = (order + 1) * (order + 2) / 2;
+    const size_t smem = sizeof(double) * n_coef * CART_STRIDE;
+    TD3_TRY(cudaFuncSetAttribute(k_cart_leaves<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem));
+    int span = cart_span(count);
+    TD3_TRY(td3_launch_chained(k_cart_leaves<P>, td3_blocks(count, span), 32 * (P + 1), smem, s,
+                               count, span, order, spos, scharge, n, center, start, end, child,
+                               moments, sdip));
+    typedef CartM2M<P> M;
+    M T{};
+    int coefs = 0;
+    for (int terms = (P + 2) * (P + 2); terms > 0; --terms)
+        for (int x = 0; x <= order; ++x)
+            for (int y = 0; x + y <= order; ++y)
+                if ((x + 1) * (y + 1) == terms) {
+                    T.x[coefs] = (unsigned char)x;
+                    T.y[coefs++] = (unsigned char)y;
+                }
+    for (i64 level = n_levels - 2; level >= 0; --level) {
+        const i64 lo = levels[level], hi = levels[level + 1];
+        if (hi <= lo) continue;
+        // consecutive nodes a block picks its parents from: a few blocks per SM, 32 at most
+        const i64 pick = (hi - lo) / (148 * 8);
+        span = pick < M::NODES ? M::NODES : pick > 32 ? 32 : (int)pick;
+        TD3_TRY(td3_launch_chained(k_cart_m2m<P>, td3_blocks(hi - lo, span), M::THREADS * M::NODES,
+                                   0, s, lo, hi, span, order, T, center, start, end, child,
+                                   moments));
+    }
+    return TD3_OK;
+}
+
 int launch_cart_moments(const int64_t* levels, int64_t n_levels, const double* spos,
                         const double* scharge, int64_t n, const double* center, const i64* start,
                         const i64* end, const i64* child, const i64* shift,
@@ -558,6 +805,14 @@ int launch_cart_moments(const int64_t* levels, int64_t n_levels, const double* s
     int order = 0;
     while ((order + 1) * (order + 2) / 2 < n_coef) ++order;
     if ((order + 1) * (order + 2) / 2 != n_coef) return TD3_EINVAL;
+#define TD3_CART_LANES(P)                                                                      \
+    return launch_cart_lanes<P>(levels, n_levels, order, spos, scharge, n, center, start, end, \
+                                child, moments, sdip, s)
+    if (order <= 4) TD3_CART_LANES(4);
+    if (order <= 8) TD3_CART_LANES(8);
+    if (order <= 12) TD3_CART_LANES(12);
+    if (order <= 16) TD3_CART_LANES(16);
+#undef TD3_CART_LANES
     unsigned threads = (unsigned)((n_coef + 31) / 32 * 32);
     if (threads > CART_MOM_THREADS) threads = CART_MOM_THREADS;
     if (n_coef > (int)threads * CART_MOM_PER_THREAD) return TD3_EINVAL;
