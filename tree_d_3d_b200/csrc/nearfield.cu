@@ -22,10 +22,13 @@ constexpr int NW_NEAR = 1;
 constexpr int LOCAL_COMPLEX = 0;
 constexpr int LOCAL_CART = 1;
 
-// Blocks of a finish launch: a warp per 32 segments, at most 148 x 16 blocks.
+// Segments a warp of the finish kernels looks at in turn (its leaves come one after another).
+constexpr int NF_SCAN = 8;
+
+// Blocks of a finish launch: a warp per NF_SCAN segments, at most 148 x 64 blocks.
 static inline unsigned td3_finish_blocks(i64 n_seg) {
-    const i64 warps = (n_seg + 31) / 32, blocks = (warps + NF_WARPS - 1) / NF_WARPS;
-    return (unsigned)(blocks < 1 ? 1 : blocks > 148 * 16 ? 148 * 16 : blocks);
+    const i64 warps = (n_seg + NF_SCAN - 1) / NF_SCAN, blocks = (warps + NF_WARPS - 1) / NF_WARPS;
+    return (unsigned)(blocks < 1 ? 1 : blocks > 148 * 64 ? 148 * 64 : blocks);
 }
 
 __device__ __forceinline__ int pow2_at_least(int v) {
@@ -481,37 +484,39 @@ __device__ __forceinline__ void finish_leaf(Targets T, i64 n_seg, const int* __r
     i64 s0 = T.start[leaf];
     int count = (int)(T.end[leaf] - s0);
     i64 nseg = leaf_segments(seg_leaf, seg, n_seg, leaf, lane);
-    // the partial sums of a target over the leaf's segments: lanes split the segments
-    // (a row can take thousands), a fixed-order warp reduction combines them
-    for (int it = 0; it < count; ++it) {
+    // lanes are (target, slice): the slices of a target split the leaf's segments (a row can
+    // take thousands) and a fixed-order reduction adds them; every target's L2P runs on its
+    // own lane (one target after another took up to 32 L2P latencies per leaf: 0.17 against
+    // 0.05 ms for the finish launch of 500k targets of 500k line charges)
+    const int tsz = pow2_at_least(count < 32 ? count : 32), slices = 32 / tsz;
+    const int ti = lane % tsz, slice = lane / tsz;
+    for (int base = 0; base < count; base += tsz) {
+        const int it = base + ti;
+        const bool valid = it < count;
         double pot = 0.0, ex = 0.0, ey = 0.0;
-        for (i64 s = seg + lane; s < seg + nseg; s += 32) {
-            i64 p = seg_out[s] + it;
-            pot += partial[3 * p];
-            ex += partial[3 * p + 1];
-            ey += partial[3 * p + 2];
+        if (valid) {
+#pragma unroll 4
+            for (i64 s = seg + slice; s < seg + nseg; s += slices) {
+                const i64 p = seg_out[s] + it;
+                pot += partial[3 * p];
+                ex += partial[3 * p + 1];
+                ey += partial[3 * p + 2];
+            }
         }
-        for (int off = 16; off > 0; off >>= 1) {
+        for (int off = tsz; off < 32; off <<= 1) {
             pot += __shfl_xor_sync(0xffffffffu, pot, off);
             ex += __shfl_xor_sync(0xffffffffu, ex, off);
             ey += __shfl_xor_sync(0xffffffffu, ey, off);
         }
-        if (ADD && lane == (it & 31)) {
-            const i64 i = T.perm[s0 + it];
-            phi[i] = POT ? pot : 0.0;
-            field[i] = ex;
-            field[T.m + i] = ey;
-        } else if (lane == (it & 31)) {
-            i64 k = s0 + it;
-            double xi = T.pos[k], yi = T.pos[T.m + k];
-            double lp, lx, ly;
-            eval_local<LOCAL>(local_a, local_b, leaf, order, width, xi - T.center[2 * leaf],
-                              yi - T.center[2 * leaf + 1], lp, lx, ly);
-            i64 i = T.perm[k];
-            phi[i] = POT ? lp + pot : 0.0;
-            field[i] = lx + ex;
-            field[T.m + i] = ly + ey;
-        }
+        if (!valid || slice != 0) continue;
+        const i64 k = s0 + it, i = T.perm[k];
+        double lp = 0.0, lx = 0.0, ly = 0.0;
+        if (!ADD)
+            eval_local<LOCAL>(local_a, local_b, leaf, order, width, T.pos[k] - T.center[2 * leaf],
+                              T.pos[T.m + k] - T.center[2 * leaf + 1], lp, lx, ly);
+        phi[i] = POT ? lp + pot : 0.0;
+        field[i] = lx + ex;
+        field[T.m + i] = ly + ey;
     }
 }
 
@@ -527,14 +532,14 @@ __global__ void k_near_finish(Targets T, i64 n_seg, const int* __restrict__ seg_
     td3_chain_wait();
     td3_chain_release();
     const int lane = threadIdx.x & 31;
-    // the first segment of a multi-segment leaf finishes it; each warp scans 32 segments
-    // at a time for them
+    // the first segment of a multi-segment leaf finishes it; each warp looks at NF_SCAN
+    // segments at a time for them
     const i64 warps = (i64)gridDim.x * NF_WARPS;
-    for (i64 base = ((i64)blockIdx.x * NF_WARPS + (threadIdx.x >> 5)) * 32; base < n_seg;
-         base += warps * 32) {
+    for (i64 base = ((i64)blockIdx.x * NF_WARPS + (threadIdx.x >> 5)) * NF_SCAN; base < n_seg;
+         base += warps * NF_SCAN) {
         const i64 mine = base + lane;
         unsigned firsts = __ballot_sync(
-            0xffffffffu, mine < n_seg && seg_out[mine] >= 0 &&
+            0xffffffffu, lane < NF_SCAN && mine < n_seg && seg_out[mine] >= 0 &&
                              (mine == 0 || seg_leaf[mine - 1] != seg_leaf[mine]));
         while (firsts) {
             const i64 seg = base + __ffs(firsts) - 1;
@@ -823,23 +828,29 @@ __device__ __forceinline__ void finish_adjoint_leaf(Targets T, Sources S, Adjoin
     i64 s0 = T.start[leaf];
     int count = (int)(T.end[leaf] - s0);
     i64 nseg = leaf_segments(seg_leaf, seg, n_seg, leaf, lane);
-    for (int it = 0; it < count; ++it) {
+    const int tsz = pow2_at_least(count < 32 ? count : 32), slices = 32 / tsz;
+    const int ti = lane % tsz, slice = lane / tsz;
+    for (int base = 0; base < count; base += tsz) {
+        const int it = base + ti;
+        const bool valid = it < count;
         double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        for (i64 s = seg + lane; s < seg + nseg; s += 32) {
-            i64 p = seg_out[s] + it;
-            for (int c = 0; c < 6; ++c) acc[c] += partial[6 * p + c];
+        if (valid) {
+#pragma unroll 2
+            for (i64 s = seg + slice; s < seg + nseg; s += slices) {
+                const i64 p = seg_out[s] + it;
+                for (int c = 0; c < 6; ++c) acc[c] += partial[6 * p + c];
+            }
         }
-        for (int c = 0; c < 6; ++c)
-            for (int off = 16; off > 0; off >>= 1)
-                acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], off);
-        if (ADD && lane == (it & 31)) {
-            adjoint_add(acc, s0 + it, T.perm[s0 + it], S.n, S, A);
-        } else if (lane == (it & 31)) {
-            i64 k = s0 + it;
+        for (int off = tsz; off < 32; off <<= 1)
+            for (int c = 0; c < 6; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], off);
+        if (!valid || slice != 0) continue;
+        const i64 k = s0 + it;
+        if (ADD)
+            adjoint_add(acc, k, T.perm[k], S.n, S, A);
+        else
             adjoint_finish<LOCAL>(acc, k, T.perm[k], S.n, S.pos[k] - T.center[2 * leaf],
                                   S.pos[S.n + k] - T.center[2 * leaf + 1], leaf, order, width,
                                   fa, fb, ba, bb, S, A);
-        }
     }
 }
 
@@ -854,11 +865,11 @@ __global__ void k_near_adjoint_finish(Targets T, Sources S, Adjoint A, i64 n_seg
     td3_chain_release();
     const int lane = threadIdx.x & 31;
     const i64 warps = (i64)gridDim.x * NF_WARPS;
-    for (i64 base = ((i64)blockIdx.x * NF_WARPS + (threadIdx.x >> 5)) * 32; base < n_seg;
-         base += warps * 32) {
+    for (i64 base = ((i64)blockIdx.x * NF_WARPS + (threadIdx.x >> 5)) * NF_SCAN; base < n_seg;
+         base += warps * NF_SCAN) {
         const i64 mine = base + lane;
         unsigned firsts = __ballot_sync(
-            0xffffffffu, mine < n_seg && seg_out[mine] >= 0 &&
+            0xffffffffu, lane < NF_SCAN && mine < n_seg && seg_out[mine] >= 0 &&
                              (mine == 0 || seg_leaf[mine - 1] != seg_leaf[mine]));
         while (firsts) {
             const i64 seg = base + __ffs(firsts) - 1;

@@ -173,8 +173,18 @@ def _m2l_coefficients(order: int, symmetric: bool) -> np.ndarray:
     return coeff
 
 
-#: partners per near-field work segment (one warp each)
-NEAR_SEGMENT = 256
+#: most partners per near-field work segment (one warp each), and about how many source
+#: particles a segment may hold: the launch ends with its longest segment (a warp's 256
+#: partners of 16 particles took 0.2 ms alone).  48k panel nodes: 1.16 -> 0.90 ms per product
+#: with 64 partners instead of 256; 50k strip charges (leaves of 32): 2.9 -> 2.6 ms with 32.
+#: Shorter ones cost the 1M-particle fields more partial sums (2 to 4 % at 16 partners).
+NEAR_SEGMENT = 64
+NEAR_SEGMENT_PARTICLES = 1024
+
+
+def _near_segment(leaf_capacity: int) -> int:
+    """Partners per near-field segment for source leaves of ``leaf_capacity``."""
+    return min(NEAR_SEGMENT, max(16, NEAR_SEGMENT_PARTICLES // leaf_capacity))
 
 #: the mixed-precision near field at the sources in three launches (td3_fmm_evaluate_mixed,
 #: td3_fmm_adjoint_mixed: far field per particle, FP32 hi + lo pair arithmetic) instead of
@@ -246,14 +256,17 @@ class _Lists(dict):
         raise KeyError(key)
 
 
-def _nearfield_plan(rows: torch.Tensor, tree, entries: int, end: torch.Tensor | None = None) -> dict:
+def _nearfield_plan(rows: torch.Tensor, tree, entries: int, end: torch.Tensor | None = None,
+                    source_capacity: int | None = None) -> dict:
     """The near-field work plan of one tree's leaf rows (td3_nearfield_plan): leaf rows
-    cut into segments of at most NEAR_SEGMENT partners, and the partial-sum buffer of
-    the rows that take several segments.  ``entries`` bounds the rows' partner count;
-    ``end`` (default the tree's node_end) set to node_start leaves a leaf out."""
+    cut into segments of partners (_near_segment of ``source_capacity``, the partners'
+    leaf capacity, by default the tree's), and the partial-sum buffer of the rows that
+    take several segments.  ``entries`` bounds the rows' partner count; ``end`` (default
+    the tree's node_end) set to node_start leaves a leaf out."""
     dev = rows.device
     n_nodes = rows.shape[0] - 1
-    capacity = n_nodes + entries // NEAR_SEGMENT + 1
+    segment = _near_segment(tree.leaf_capacity if source_capacity is None else source_capacity)
+    capacity = n_nodes + entries // segment + 1
     seg_leaf = torch.empty(capacity, dtype=torch.int32, device=dev)
     seg_range = torch.empty((capacity, 2), dtype=torch.int64, device=dev)
     seg_out = torch.empty(capacity, dtype=torch.int64, device=dev)
@@ -261,7 +274,7 @@ def _nearfield_plan(rows: torch.Tensor, tree, entries: int, end: torch.Tensor | 
     ws = _lib.workspace(_lib.query("td3_nearfield_plan_workspace_size", n_nodes), dev)
     end = tree.node_end if end is None else end
     _lib.call("td3_nearfield_plan", rows.data_ptr(), n_nodes, tree.node_child.data_ptr(),
-              tree.node_start.data_ptr(), end.data_ptr(), NEAR_SEGMENT,
+              tree.node_start.data_ptr(), end.data_ptr(), segment,
               seg_leaf.data_ptr(), seg_range.data_ptr(), seg_out.data_ptr(), capacity,
               sizes.ctypes.data, ws.data_ptr(), ws.numel(), _lib.stream(dev))
     n_seg = int(sizes[0])
@@ -1161,7 +1174,8 @@ class FlatQuadtree:
         return {
             "m2l": m2l, "p2p": p2p, "m2l_rows": m2l_rows, "m2l_partners": m2l_partners,
             "m2l_entry_row": m2l_entry, "p2p_rows": p2p_rows, "p2p_partners": p2p_partners,
-            "plan": _nearfield_plan(p2p_rows, tree, p2p.shape[0]),
+            "plan": _nearfield_plan(p2p_rows, tree, p2p.shape[0],
+                                    source_capacity=self.leaf_capacity),
         }
 
     def _target_plan(self, targets: torch.Tensor, theta: float, leaf: int):
