@@ -7,9 +7,10 @@
 //   pair_csr       pair lists as rows by node (K/pair_csr/pair_csr_pyccel.py:12-45).
 //
 // A generation classifies every frontier pair (M2L, P2P, its 4 or 10 child pairs, or
-// dropped), an exclusive scan of the per-pair counts gives each output its slot, and a
-// second pass writes them: the lists come out in the reference's serial order.  The
-// frontier sizes stay on the device; the host looks at them every few generations.  The
+// dropped) and writes each output to its slot in one launch: the tiles of the frontier get
+// their first slots from the tiles before them (decoupled look-back), so the lists come out
+// in the reference's serial order.  The frontier sizes stay on the device; the host looks at
+// them every few generations.  The
 // predicates use exactly rounded operations (this file is compiled with --fmad=false).
 #include "common.cuh"
 
@@ -64,18 +65,6 @@ __device__ __forceinline__ int classify_mutual(i64 a, i64 b, const NodeRec* __re
     return ACT_SPLIT_B;
 }
 
-// counts: a = m2l | (p2p << 32), b = next-frontier pairs
-__device__ __forceinline__ td3_i64x2 action_counts(int act) {
-    switch (act) {
-        case ACT_M2L: return td3_i64x2(1, 0);
-        case ACT_P2P: return td3_i64x2((i64)1 << 32, 0);
-        case ACT_SELF: return td3_i64x2(0, 10);
-        case ACT_SPLIT_A:
-        case ACT_SPLIT_B: return td3_i64x2(0, 4);
-        default: return td3_i64x2(0, 0);
-    }
-}
-
 // The one-way decision for (target cell a, source cell b) (dual_traverse_pyccel.py:46-86).
 __device__ __forceinline__ int classify_dual(i64 a, i64 b, const NodeRec* __restrict__ t_rec,
                                              const NodeRec* __restrict__ s_rec, double theta) {
@@ -92,23 +81,43 @@ __device__ __forceinline__ int classify_dual(i64 a, i64 b, const NodeRec* __rest
 }
 
 // ------------------------------------------------------------------ generations
-// A generation is three launches of fixed size that read the frontier size from device
-// memory: classify (action per pair, counts per tile of GEN_TILE pairs), an exclusive
-// scan of the tile counts (one block; it also checks the buffers and advances the
-// totals), and emit (per tile, block scans of the pairs' counts in frontier order give
-// every output its slot).  The host reads the state once per GEN_BATCH generations.
-constexpr int GEN_ITEMS = 8;
+// A generation is one launch that reads the frontier size from device memory.  Its blocks
+// take tiles of GEN_TILE pairs in order (a ticket each); a tile's pairs are classified once,
+// with their actions in registers, its counts published, and its first slots found from the
+// tiles before it: their counts up to the nearest one whose own first slots are known
+// (Merrill and Garland's decoupled look-back).  Tiles are taken in order by resident blocks,
+// so a tile's predecessors are always under way; the wait for them is bounded all the same
+// (LOOK_LIMIT polls, then the state's `failed`, which the host turns into an error).
+//
+// Measured (all generations of theta 0.5, host reads included) against two launches per
+// generation, one that classifies and scans and one that reads the frontier again and emits:
+// 0.84 -> 0.50 ms (1M clustered particles, leaf 8), 0.51 -> 0.28 ms (200k), 0.24 -> 0.13 ms
+// (2000).  GEN_ITEMS 8 (fewer, longer tiles) 0.53 / 0.36 / 0.16 ms, 2: 0.61 / 0.30 / 0.12 ms.
+constexpr int GEN_ITEMS = 4;
 constexpr int GEN_TILE = TRAV_THREADS * GEN_ITEMS;
-constexpr int GEN_BATCH = 8;
+constexpr int GEN_FIRST = 16, GEN_BATCH = 8;  // generations before the first / next host read
+constexpr int GEN_BLOCKS = 4;  // resident per SM
+constexpr unsigned LOOK_LIMIT = 1u << 22;
 
 struct TravState {
     i64 nf[2];          // frontier size of even / odd generations
-    i64 emit_nf;        // frontier size the current emit pass writes (0 after overflow)
     i64 n_m2l, n_p2p;   // pairs listed so far
-    i64 base_m2l, base_p2p;
     i64 overflow;       // a list or the next frontier outgrew its buffer
     i64 need_m2l, need_p2p, need_frontier;
-    unsigned long long arrived;  // classify blocks done in the current generation
+    i64 failed;         // a wait ran out
+    unsigned ticket[4];  // tiles taken, of generation g at g mod 4
+};
+
+// A tile's counts of a generation (its own, or with all tiles before it): m2l and p2p pairs
+// in the halves of `lists`, next-frontier pairs in `next`.  `ready` is 2 g + 1 once `own` is
+// there and 2 g + 2 once `all` is, g the generation's number from 0.
+struct TileCounts {
+    unsigned long long lists;
+    unsigned long long next;
+};
+struct TileState {
+    TileCounts own, all;
+    unsigned ready, pad[3];
 };
 
 template <bool DUAL>
@@ -118,190 +127,230 @@ __device__ __forceinline__ int classify_pair(const NodeRec* t, const NodeRec* s,
     return classify_mutual(pr.a, pr.b, t, theta);
 }
 
-__device__ __forceinline__ td3_i64x2 warp_inclusive_x2(td3_i64x2 v, int lane) {
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        long long a = __shfl_up_sync(0xffffffffu, (long long)v.a, d);
-        long long b = __shfl_up_sync(0xffffffffu, (long long)v.b, d);
-        if (lane >= d) {
-            v.a += a;
-            v.b += b;
-        }
-    }
-    return v;
-}
-
-// Exclusive scan over the block (blockDim.x a multiple of 32, at most 1024 threads).
-__device__ __forceinline__ td3_i64x2 block_exclusive_x2(td3_i64x2 v, td3_i64x2* total) {
-    __shared__ td3_i64x2 sums[32];
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    td3_i64x2 inc = warp_inclusive_x2(v, lane);
-    if (lane == 31) sums[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-        td3_i64x2 x = lane < nw ? sums[lane] : td3_i64x2(0);
-        x = warp_inclusive_x2(x, lane);
-        if (lane < nw) sums[lane] = x;
-    }
-    __syncthreads();
-    td3_i64x2 off = warp ? sums[warp - 1] : td3_i64x2(0);
-    *total = sums[nw - 1];
-    __syncthreads();
-    return off + inc - v;
-}
-
-__global__ void k_gen_init(TravState* st, FPair* frontier) {
+__global__ void k_gen_init(TravState* st, FPair* frontier, TileState* tile, i64 tiles) {
     td3_chain_wait();
     td3_chain_release();
+    const i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < tiles) tile[i].ready = 0;
+    if (i) return;
+    *st = TravState{};
     st->nf[0] = 1;
-    st->nf[1] = 0;
-    st->emit_nf = 0;
-    st->n_m2l = st->n_p2p = st->base_m2l = st->base_p2p = 0;
-    st->overflow = st->need_m2l = st->need_p2p = st->need_frontier = 0;
-    st->arrived = 0;
     frontier[0] = FPair{0, 0};
 }
 
-template <bool DUAL>
-__global__ void __launch_bounds__(TRAV_THREADS)
-k_gen_classify(const FPair* __restrict__ frontier, TravState* st, int parity,
-               const NodeRec* __restrict__ t, const NodeRec* __restrict__ s, double theta,
-               signed char* __restrict__ action, td3_i64x2* __restrict__ tile_sum,
-               i64 m2l_capacity, i64 p2p_capacity, i64 frontier_capacity) {
-    __shared__ bool last;
-    td3_chain_wait();
-    td3_chain_release();
-    i64 nf = st->nf[parity];
-    i64 tiles = (nf + GEN_TILE - 1) / GEN_TILE;
-    for (i64 tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        td3_i64x2 sum(0);
-#pragma unroll
-        for (int i = 0; i < GEN_ITEMS; ++i) {
-            i64 k = tile * GEN_TILE + i * TRAV_THREADS + threadIdx.x;
-            if (k < nf) {
-                int act = classify_pair<DUAL>(t, s, theta, frontier[k]);
-                action[k] = (signed char)act;
-                sum += action_counts(act);
-            }
-        }
-        td3_i64x2 total;
-        block_exclusive_x2(sum, &total);
-        if (threadIdx.x == 0) tile_sum[tile] = total;
-    }
-    // The last block to finish scans the tile sums (no block waits: the others leave).
-    if (threadIdx.x == 0) {
-        __threadfence();  // this block's tile sums before its arrival
-        last = atomicAdd(&st->arrived, 1ull) == (unsigned long long)gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    td3_i64x2 carry(0);
-    for (i64 c = 0; c < tiles; c += blockDim.x) {
-        i64 tile = c + threadIdx.x;
-        td3_i64x2 v(0);
-        if (tile < tiles) {
-            v.a = __ldcg(reinterpret_cast<const long long*>(&tile_sum[tile].a));
-            v.b = __ldcg(reinterpret_cast<const long long*>(&tile_sum[tile].b));
-        }
-        td3_i64x2 total;
-        td3_i64x2 ex = block_exclusive_x2(v, &total);
-        if (tile < tiles) tile_sum[tile] = carry + ex;
-        carry += total;
-    }
-    if (threadIdx.x == 0) {
-        st->arrived = 0;
-        i64 add_m2l = carry.a & 0xffffffffLL, add_p2p = carry.a >> 32, nn = carry.b;
-        st->base_m2l = st->n_m2l;
-        st->base_p2p = st->n_p2p;
-        if (st->n_m2l + add_m2l > m2l_capacity || st->n_p2p + add_p2p > p2p_capacity ||
-            nn > frontier_capacity) {
-            st->overflow = 1;
-            st->need_m2l = st->n_m2l + add_m2l;
-            st->need_p2p = st->n_p2p + add_p2p;
-            st->need_frontier = nn;
-            st->emit_nf = 0;
-            st->nf[parity ^ 1] = 0;
-        } else {
-            st->n_m2l += add_m2l;
-            st->n_p2p += add_p2p;
-            st->emit_nf = nf;
-            st->nf[parity ^ 1] = nn;
-        }
-    }
+__device__ __forceinline__ unsigned load_acquire(const unsigned* p) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void store_release(unsigned* p, unsigned v) {
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Emit: a warp takes 32 * GEN_ITEMS consecutive pairs of the tile (round r, lane l:
-// pair warp_base + 32 r + l); the warps' totals are scanned once per tile, then each
-// round's slots come from a warp scan, in frontier order.
+// The counts of all tiles before `tile` (one warp; every lane returns them): 32 tiles at a
+// time, the lanes nearest first, up to the nearest tile whose `all` is there.
+__device__ TileCounts look_back(TileState* state, i64 tile, unsigned own_ready, bool* failed) {
+    const int lane = threadIdx.x & 31;
+    TileCounts sum{0, 0};
+    for (i64 at = tile - 1; at >= 0; at -= 32) {
+        const i64 t = at - lane;
+        unsigned ready = own_ready + 1;  // before the first tile: nothing, known
+        if (t >= 0) {
+            unsigned polls = 0;
+            while ((ready = load_acquire(&state[t].ready)) < own_ready && ++polls < LOOK_LIMIT)
+                __nanosleep(20);
+        }
+        if (__any_sync(0xffffffffu, ready < own_ready)) {
+            *failed = true;
+            return sum;
+        }
+        const unsigned known = __ballot_sync(0xffffffffu, ready > own_ready);
+        const int last = known ? __ffs(known) - 1 : 31;  // the nearest tile with `all`
+        TileCounts c{0, 0};
+        if (t >= 0 && lane <= last) {
+            const TileCounts* from = lane == last && known ? &state[t].all : &state[t].own;
+            c.lists = __ldcg(&from->lists);
+            c.next = __ldcg(&from->next);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            c.lists += __shfl_xor_sync(0xffffffffu, c.lists, o);
+            c.next += __shfl_xor_sync(0xffffffffu, c.next, o);
+        }
+        sum.lists += c.lists;
+        sum.next += c.next;
+        if (known) break;
+    }
+    return sum;
+}
+
+// One generation.  A warp takes 32 * GEN_ITEMS consecutive pairs of a tile (round r, lane l:
+// pair first + 32 r + l); ballots rank a round's outputs, in frontier order.
 template <bool DUAL>
-__global__ void __launch_bounds__(TRAV_THREADS)
-k_gen_emit(const FPair* __restrict__ frontier, const TravState* st,
-           const signed char* __restrict__ action, const td3_i64x2* __restrict__ tile_off,
-           const NodeRec* __restrict__ t_rec, const NodeRec* __restrict__ s_rec,
-           Pair* __restrict__ m2l, Pair* __restrict__ p2p, FPair* __restrict__ next) {
-    __shared__ td3_i64x2 warp_total[TRAV_THREADS / 32];
+__global__ void __launch_bounds__(TRAV_THREADS, GEN_BLOCKS)
+k_generation(const FPair* __restrict__ frontier, TravState* st, int gen,
+             const NodeRec* __restrict__ t_rec, const NodeRec* __restrict__ s_rec, double theta,
+             TileState* tile_state, Pair* __restrict__ m2l, i64 m2l_capacity,
+             Pair* __restrict__ p2p, i64 p2p_capacity, FPair* __restrict__ next,
+             i64 frontier_capacity) {
+    constexpr int WARPS = TRAV_THREADS / 32;
+    __shared__ unsigned warp_m2l[WARPS], warp_p2p[WARPS], warp_next[WARPS];
+    __shared__ i64 base_m2l_s, base_p2p_s, base_next_s;
+    __shared__ unsigned taken;
     td3_chain_wait();
     td3_chain_release();
-    int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    i64 nf = st->emit_nf;
-    i64 base_m2l = st->base_m2l, base_p2p = st->base_p2p;
-    i64 tiles = (nf + GEN_TILE - 1) / GEN_TILE;
-    for (i64 tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        i64 first = tile * GEN_TILE + (i64)wib * 32 * GEN_ITEMS;
-        int act[GEN_ITEMS];
-        td3_i64x2 mine(0);
-#pragma unroll
-        for (int r = 0; r < GEN_ITEMS; ++r) {
-            i64 k = first + r * 32 + lane;
-            act[r] = k < nf ? action[k] : ACT_NONE;
-            mine += action_counts(act[r]);
-        }
-        td3_i64x2 wsum = warp_inclusive_x2(mine, lane);
-        __syncthreads();  // the previous tile's readers are done with warp_total
-        if (lane == 31) warp_total[wib] = wsum;
+    const int parity = gen & 1, lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const unsigned before = (1u << lane) - 1u;
+    // read before this block takes a tile: the last tile's block moves them on (a generation
+    // after a failed one, whose frontier has holes, is empty)
+    const i64 nf = st->failed ? 0 : st->nf[parity], listed_m2l = st->n_m2l, listed_p2p = st->n_p2p;
+    const i64 tiles = (nf + GEN_TILE - 1) / GEN_TILE;
+    const unsigned own_ready = 2u * (unsigned)gen + 1u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        st->ticket[(gen + 2) & 3] = 0;
+        if (tiles == 0) st->nf[parity ^ 1] = 0;
+    }
+    if ((i64)blockIdx.x >= tiles) return;  // the others take every tile
+    for (;;) {
+        if (threadIdx.x == 0) taken = atomicAdd(&st->ticket[gen & 3], 1u);
         __syncthreads();
-        td3_i64x2 carry = tile_off[tile];
-        for (int w = 0; w < wib; ++w) carry += warp_total[w];
+        const i64 tile = taken;
+        if (tile >= tiles) return;
+        const i64 first = tile * GEN_TILE + (i64)wib * 32 * GEN_ITEMS;
+        FPair pr[GEN_ITEMS];
+        int act[GEN_ITEMS];
+        unsigned n_m2l = 0, n_p2p = 0, n_next = 0;  // the warp's
 #pragma unroll
         for (int r = 0; r < GEN_ITEMS; ++r) {
-            td3_i64x2 c = action_counts(act[r]);
-            td3_i64x2 inc = warp_inclusive_x2(c, lane);
-            td3_i64x2 off = carry + inc - c;
-            long long ta = __shfl_sync(0xffffffffu, (long long)inc.a, 31);
-            long long tb = __shfl_sync(0xffffffffu, (long long)inc.b, 31);
-            carry += td3_i64x2(ta, tb);
-            if (act[r] == ACT_NONE) continue;
-            FPair pr = frontier[first + r * 32 + lane];
+            const i64 k = first + r * 32 + lane;
+            pr[r] = k < nf ? frontier[k] : FPair{0, 0};
+        }
+#pragma unroll
+        for (int r = 0; r < GEN_ITEMS; ++r) {
+            const i64 k = first + r * 32 + lane;
+            act[r] = k < nf ? classify_pair<DUAL>(t_rec, s_rec, theta, pr[r]) : ACT_NONE;
+        }
+#pragma unroll
+        for (int r = 0; r < GEN_ITEMS; ++r) {
+            n_m2l += __popc(__ballot_sync(0xffffffffu, act[r] == ACT_M2L));
+            n_p2p += __popc(__ballot_sync(0xffffffffu, act[r] == ACT_P2P));
+            n_next += 4 * __popc(__ballot_sync(0xffffffffu, act[r] >= ACT_SPLIT_A));
+            if (!DUAL) n_next += 10 * __popc(__ballot_sync(0xffffffffu, act[r] == ACT_SELF));
+        }
+        if (lane == 0) {
+            warp_m2l[wib] = n_m2l;
+            warp_p2p[wib] = n_p2p;
+            warp_next[wib] = n_next;
+        }
+        __syncthreads();
+        if (wib == 0) {
+            // the tile's counts, published; then the tiles' before it
+            TileCounts own{0, 0};
+            for (int w = 0; w < WARPS; ++w) {
+                own.lists += warp_m2l[w] | ((unsigned long long)warp_p2p[w] << 32);
+                own.next += warp_next[w];
+            }
+            TileState* mine = tile_state + tile;
+            if (lane == 0 && tile) {
+                __stcg(&mine->own.lists, own.lists);
+                __stcg(&mine->own.next, own.next);
+                store_release(&mine->ready, own_ready);
+            }
+            bool failed = false;
+            const TileCounts pre = look_back(tile_state, tile, own_ready, &failed);
+            if (lane == 0) {
+                const TileCounts all{pre.lists + own.lists, pre.next + own.next};
+                if (failed) {
+                    st->failed = 1;
+                    st->nf[parity ^ 1] = 0;
+                    taken = 0xffffffffu;
+                } else {
+                    __stcg(&mine->all.lists, all.lists);
+                    __stcg(&mine->all.next, all.next);
+                    store_release(&mine->ready, own_ready + 1);
+                    base_m2l_s = listed_m2l + (i64)(pre.lists & 0xffffffffull);
+                    base_p2p_s = listed_p2p + (i64)(pre.lists >> 32);
+                    base_next_s = (i64)pre.next;
+                    if (tile == tiles - 1) {
+                        const i64 total_m2l = listed_m2l + (i64)(all.lists & 0xffffffffull);
+                        const i64 total_p2p = listed_p2p + (i64)(all.lists >> 32);
+                        const i64 nn = (i64)all.next;
+                        if (total_m2l > m2l_capacity || total_p2p > p2p_capacity ||
+                            nn > frontier_capacity) {
+                            st->overflow = 1;
+                            st->need_m2l = total_m2l;
+                            st->need_p2p = total_p2p;
+                            st->need_frontier = nn;
+                            st->nf[parity ^ 1] = 0;
+                        } else {
+                            st->n_m2l = total_m2l;
+                            st->n_p2p = total_p2p;
+                            st->nf[parity ^ 1] = nn;
+                        }
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        if (taken == 0xffffffffu) return;
+        i64 at_m2l = base_m2l_s, at_p2p = base_p2p_s, at_next = base_next_s;
+        for (int w = 0; w < wib; ++w) {
+            at_m2l += warp_m2l[w];
+            at_p2p += warp_p2p[w];
+            at_next += warp_next[w];
+        }
+#pragma unroll
+        for (int r = 0; r < GEN_ITEMS; ++r) {
+            const unsigned bm = __ballot_sync(0xffffffffu, act[r] == ACT_M2L);
+            const unsigned bp = __ballot_sync(0xffffffffu, act[r] == ACT_P2P);
+            const unsigned bs = __ballot_sync(0xffffffffu, act[r] >= ACT_SPLIT_A);
+            const unsigned bb = DUAL ? 0u : __ballot_sync(0xffffffffu, act[r] == ACT_SELF);
+            const i64 to = at_next + 4 * __popc(bs & before) + 10 * __popc(bb & before);
+            // outputs past a buffer's end are left out: the last tile reports the overflow
             switch (act[r]) {
-                case ACT_M2L: m2l[base_m2l + (off.a & 0xffffffffLL)] = Pair{pr.a, pr.b}; break;
-                case ACT_P2P: p2p[base_p2p + (off.a >> 32)] = Pair{pr.a, pr.b}; break;
+                case ACT_NONE: break;
+                case ACT_M2L: {
+                    const i64 j = at_m2l + __popc(bm & before);
+                    if (j < m2l_capacity) m2l[j] = Pair{pr[r].a, pr[r].b};
+                    break;
+                }
+                case ACT_P2P: {
+                    const i64 j = at_p2p + __popc(bp & before);
+                    if (j < p2p_capacity) p2p[j] = Pair{pr[r].a, pr[r].b};
+                    break;
+                }
                 case ACT_SELF: {
-                    int f = t_rec[pr.a].child;
-                    i64 j = off.b;
+                    if (to + 10 > frontier_capacity) break;
+                    const int f = t_rec[pr[r].a].child;
+                    i64 j = to;
                     for (int c1 = 0; c1 < 4; ++c1)
                         for (int d = c1; d < 4; ++d) next[j++] = FPair{f + c1, f + d};
                     break;
                 }
                 case ACT_SPLIT_A: {
-                    int f = t_rec[pr.a].child;
-                    for (int c1 = 0; c1 < 4; ++c1) next[off.b + c1] = FPair{f + c1, pr.b};
+                    if (to + 4 > frontier_capacity) break;
+                    const int f = t_rec[pr[r].a].child;
+                    for (int c1 = 0; c1 < 4; ++c1) next[to + c1] = FPair{f + c1, pr[r].b};
                     break;
                 }
                 default: {
-                    int f = (DUAL ? s_rec : t_rec)[pr.b].child;
-                    for (int c1 = 0; c1 < 4; ++c1) next[off.b + c1] = FPair{pr.a, f + c1};
+                    if (to + 4 > frontier_capacity) break;
+                    const int f = (DUAL ? s_rec : t_rec)[pr[r].b].child;
+                    for (int c1 = 0; c1 < 4; ++c1) next[to + c1] = FPair{pr[r].a, f + c1};
                     break;
                 }
             }
+            at_m2l += __popc(bm);
+            at_p2p += __popc(bp);
+            at_next += 4 * __popc(bs) + 10 * __popc(bb);
         }
+        __syncthreads();  // the tile's counts and slots have been read
     }
 }
 
 struct TraverseBuffers {
     FPair* frontier[2];
-    signed char* action;
-    td3_i64x2* tile_sum;
+    TileState* tile;
     TravState* state;
     NodeRec* rec[2];  // target (and source) tree records
 };
@@ -309,16 +358,15 @@ struct TraverseBuffers {
 i64 gen_tiles(i64 frontier_cap) { return (frontier_cap + GEN_TILE - 1) / GEN_TILE; }
 
 size_t traverse_workspace(i64 frontier_cap, i64 n_records) {
-    return 2 * td3_ws_bytes<FPair>(frontier_cap) + td3_ws_bytes<signed char>(frontier_cap) +
-           td3_ws_bytes<td3_i64x2>(gen_tiles(frontier_cap)) + td3_ws_bytes<TravState>(1) +
+    return 2 * td3_ws_bytes<FPair>(frontier_cap) +
+           td3_ws_bytes<TileState>(gen_tiles(frontier_cap)) + td3_ws_bytes<TravState>(1) +
            td3_ws_bytes<NodeRec>(n_records) + 512;
 }
 
 bool take_traverse(Workspace& w, i64 frontier_cap, i64 n_t, i64 n_s, TraverseBuffers& b) {
     b.frontier[0] = w.take<FPair>(frontier_cap);
     b.frontier[1] = w.take<FPair>(frontier_cap);
-    b.action = w.take<signed char>(frontier_cap);
-    b.tile_sum = w.take<td3_i64x2>(gen_tiles(frontier_cap));
+    b.tile = w.take<TileState>(gen_tiles(frontier_cap));
     b.state = w.take<TravState>(1);
     b.rec[0] = w.take<NodeRec>(n_t);
     b.rec[1] = n_s ? w.take<NodeRec>(n_s) : b.rec[0];
@@ -340,26 +388,26 @@ int run_generations(const NodeRec* t, const NodeRec* s, double theta, Pair* m2l,
                     int64_t* sizes, const TraverseBuffers& b, cudaStream_t stream) {
     i64 tiles = gen_tiles(frontier_capacity);
     unsigned grid = (unsigned)(tiles < 148 * 4 ? tiles : 148 * 4);
-    TD3_TRY(td3_launch_chained(k_gen_init, 1, 1, 0, stream, b.state, b.frontier[0]));
+    TD3_TRY(td3_launch_chained(k_gen_init, td3_blocks(tiles, 256), 256, 0, stream, b.state,
+                               b.frontier[0], b.tile, tiles));
     TD3_CHECK_LAUNCH();
     sizes[0] = sizes[1] = sizes[2] = sizes[3] = 0;
     for (int gen = 0;;) {
-        for (int k = 0; k < GEN_BATCH; ++k, ++gen) {
-            int parity = gen & 1;
-            TD3_TRY(td3_launch_chained(k_gen_classify<DUAL>, grid, TRAV_THREADS, 0, stream,
-                                       (const FPair*)b.frontier[parity], b.state, parity, t, s,
-                                       theta, b.action, b.tile_sum, m2l_capacity, p2p_capacity,
-                                       frontier_capacity));
-            TD3_TRY(td3_launch_chained(k_gen_emit<DUAL>, grid, TRAV_THREADS, 0, stream,
-                                       (const FPair*)b.frontier[parity], (const TravState*)b.state,
-                                       (const signed char*)b.action,
-                                       (const td3_i64x2*)b.tile_sum, t, s, m2l, p2p,
-                                       b.frontier[parity ^ 1]));
-            TD3_CHECK_LAUNCH();
+        for (const int stop = gen + (gen ? GEN_BATCH : GEN_FIRST); gen < stop; ++gen) {
+            const int parity = gen & 1;
+            TD3_TRY(td3_launch_chained(k_generation<DUAL>, grid, TRAV_THREADS, 0, stream,
+                                       (const FPair*)b.frontier[parity], b.state, gen, t, s,
+                                       theta, b.tile, m2l, m2l_capacity, p2p, p2p_capacity,
+                                       b.frontier[parity ^ 1], frontier_capacity));
         }
+        TD3_CHECK_LAUNCH();
         TravState h;
         TD3_TRY(cudaMemcpyAsync(&h, b.state, sizeof(h), cudaMemcpyDeviceToHost, stream));
         TD3_TRY(cudaStreamSynchronize(stream));
+        if (h.failed) {
+            td3_set_error("a generation of the traversal did not complete (a bounded wait ran out)");
+            return TD3_ECUDA;
+        }
         if (h.overflow) {
             sizes[0] = h.need_m2l;
             sizes[1] = h.need_p2p;
