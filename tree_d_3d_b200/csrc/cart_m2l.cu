@@ -20,29 +20,19 @@
 // operands in shared memory, FP32 4.5 ms (100k particles, two launches of the backward
 // step: 2.3 -> 0.9 ms).
 //
-// Work: a warp owns a run of whole destination rows (an even share of entries + a cost per
-// row).  Its eight 4-lane groups take the rows in order; lane i of a group translates
-// entries i, i + 4, ... and keeps its sums across the row.  At the row's end the group's 4
-// lanes are added through shared memory and each lane adds a quarter of the coefficients to
-// the locals.  (Groups of 4: a row of 35 entries, the mean at theta 0.5,
-// fills 97 % of its lanes' rounds against 87 % with 8.)  Rows above LONG_ROW entries are
-// taken by the whole warp first.  Each row is summed by one group or warp in a fixed
-// order: the same bits every run.
+// Work: a warp walks its rows with four lanes per row (walk_rows); a lane keeps its sums
+// across the row, at whose end the group's 4 lanes are added through shared memory and each
+// lane adds a quarter of the coefficients to the locals: the same bits every run.
 //
 // Mixed precision (T = float): moments in units of the source cell's half-width h_s and
 // sums in units of the destination's h_d; see translate().
-#include "common.cuh"
+#include "row_groups.cuh"
 
 #include <type_traits>
 #include <utility>
 
 namespace {
 
-constexpr int GL = 4;            // lanes per destination row
-constexpr int GROUPS = 32 / GL;  // rows in flight per warp
-constexpr int LONG_ROW = 256;    // rows longer than this are taken by the whole warp
-constexpr int ROW_COST = 8;      // entries a row counts for in the warps' shares
-constexpr unsigned FULL = 0xffffffffu;
 constexpr int MAX_DEVICES = 64;
 
 __host__ __device__ constexpr int tri(int n) { return n * (n + 1) / 2; }
@@ -109,9 +99,6 @@ struct CartScale {
     double inv_fact2[tri(17)];
 };
 
-__device__ __forceinline__ unsigned shared_address(const void* p) {
-    return (unsigned)__cvta_generic_to_shared(p);
-}
 // 16 bytes to shared memory, zeros without `on` (nothing is then read).
 __device__ __forceinline__ void copy16(unsigned smem, const void* global, bool on) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem), "l"(global),
@@ -121,10 +108,6 @@ __device__ __forceinline__ void copy16(unsigned smem, const void* global, bool o
 __device__ __forceinline__ void prefetch_l2(const void* global, int bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(global), "r"(bytes));
 }
-__device__ __forceinline__ void copies_done() {
-    asm volatile("cp.async.wait_all;" ::: "memory");
-}
-
 template <typename T>
 constexpr bool PAIR = sizeof(T) == 4;
 
@@ -362,25 +345,9 @@ k_m2l_cart_rows(const i64* __restrict__ row_start, const i64* __restrict__ partn
     extern __shared__ __align__(16) char cart_smem[];
     td3_chain_wait();
     td3_chain_release();
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, g = lane / GL, gl = lane % GL;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, gl = lane % ROW_GL;
     T* stage = reinterpret_cast<T*>(cart_smem) + (size_t)wib * 32 * PITCH_S;
     const int n_coef = tri(order + 1);
-
-    const i64 gw = (i64)blockIdx.x * WARPS_PER_BLOCK<T> + wib;
-    const i64 nw = (i64)gridDim.x * WARPS_PER_BLOCK<T>;
-    const i64 total = row_start[n_dst] + ROW_COST * n_dst, share = (total + nw - 1) / nw;
-    auto first_row_at = [&](i64 c) {
-        i64 lo = 0, hi = n_dst;
-        while (lo < hi) {
-            i64 mid = (lo + hi) >> 1;
-            if (row_start[mid] + ROW_COST * mid < c) lo = mid + 1;
-            else hi = mid;
-        }
-        return lo;
-    };
-    const i64 da = first_row_at(gw * share);
-    const i64 db = gw + 1 == nw ? n_dst : first_row_at((gw + 1) * share);
-    if (da >= db) return;
 
     constexpr int NC = compensated<T, B0>(NB);
     T acc[NB + NC];
@@ -388,8 +355,19 @@ k_m2l_cart_rows(const i64* __restrict__ row_start, const i64* __restrict__ partn
     for (int k = 0; k < NB + NC; ++k) acc[k] = T(0);
 
     // The moments of the lanes' partners (src < 0: none) into the lanes' rows of `stage`
-    // (packed: copies in flight until copies_done()).
-    auto fetch = [&](int src) {
+    // (packed: copies in flight until copies_done()), and the translations and sizes.
+    double tx = 0.0, ty = 0.0, hs = 0.0, hd = 1.0;
+    auto fetch = [&](int src, i64 d) {
+        if (src >= 0) {
+            const double2 c = reinterpret_cast<const double2*>(src_center)[src];
+            const double2 cd = reinterpret_cast<const double2*>(dst_center)[d];
+            tx = cd.x - c.x;
+            ty = cd.y - c.y;
+            if (MIXED) {
+                hs = src_half[src];
+                hd = dst_half[d];
+            }
+        }
         __syncwarp();
         if (packed) {
             // the 32 x W words in turn, 32 at a time: consecutive lanes take consecutive words
@@ -398,7 +376,7 @@ k_m2l_cart_rows(const i64* __restrict__ row_start, const i64* __restrict__ partn
             int p = lane / W, w = lane % W;  // record and word of this lane
 #pragma unroll 8
             for (int k = 0; k < W; ++k) {
-                const int s = __shfl_sync(FULL, src, p);
+                const int s = __shfl_sync(FULL_WARP, src, p);
                 copy16(to + (unsigned)(p * PITCH_S * sizeof(T)) + 16 * w,
                        rec + (size_t)(s < 0 ? 0 : s) * (16 * WORDS<T, P>) + 16 * w, s >= 0);
                 p += 32 / W;
@@ -411,7 +389,7 @@ k_m2l_cart_rows(const i64* __restrict__ row_start, const i64* __restrict__ partn
         } else {
             const double* mom = static_cast<const double*>(source);
             for (int p = 0; p < 32; ++p) {
-                const int s = __shfl_sync(FULL, src, p);
+                const int s = __shfl_sync(FULL_WARP, src, p);
                 if (s < 0) continue;
                 const double inv_h = MIXED ? 1.0 / src_half[s] : 1.0;
                 for (int a = lane; a < n_coef && a < tri(NA + 1); a += 32) {
@@ -436,7 +414,7 @@ k_m2l_cart_rows(const i64* __restrict__ row_start, const i64* __restrict__ partn
 #pragma unroll
         for (int k = 0; k < NB; ++k) own[k] = k < NC ? acc[k] - acc[NB + k] : acc[k];
         __syncwarp(mask);
-        const T* rows = stage + (lane & ~(GL - 1)) * PITCH_S + first;
+        const T* rows = stage + (lane & ~(ROW_GL - 1)) * PITCH_S + first;
 #pragma unroll
         for (int k = 0; k < Q; ++k) {
             sum[k] = T(0);
@@ -470,109 +448,31 @@ k_m2l_cart_rows(const i64* __restrict__ row_start, const i64* __restrict__ partn
         }
     };
 
-    // Rows above LONG_ROW entries first, the whole warp on each (lane i at entries i, i + 32,
-    // ...), then the others, a group on each, the groups taking the rows in order.
-    i64 scan = da;        // long rows are looked for from `scan` on, 32 rows at a time
-    unsigned longs = 0;   // those found in the 32 rows before `scan`
-    auto next_long = [&]() -> i64 {
-        while (!longs && scan < db) {
-            const i64 r = scan + lane;
-            longs = __ballot_sync(FULL, r < db && row_start[r + 1] - row_start[r] > LONG_ROW);
-            scan += 32;
-        }
-        if (!longs) return -1;
-        const int k = __ffs(longs) - 1;
-        longs &= longs - 1;
-        return scan - 32 + k;
-    };
-    // A lane's place: destination row da + d (d < 0: none), entries e0 + cur, ... of it left
-    // (32-bit distances from the warp's first row and entry).
-    const i64 e0 = row_start[da];
-    struct Place {
-        int d, cur, end;
-        bool filled;  // the row has entries to sum here
-    };
-    auto claim = [&](i64 row, bool whole) {
-        Place at{row < db ? (int)(row - da) : -1, 0, 0, false};
-        if (at.d < 0) return at;
-        const int start = (int)(row_start[row] - e0);
-        at.cur = start + (whole ? lane : gl);
-        at.end = (int)(row_start[row + 1] - e0);
-        if (!whole && at.end - start > LONG_ROW) at.end = start;  // done as a long row
-        at.filled = at.end > start;
-        return at;
-    };
-    auto partner = [&](const Place& at) {
-        return at.d >= 0 && at.cur < at.end ? (int)partners[e0 + at.cur] : -1;
-    };
-    i64 next = da + GROUPS;  // the first row that no group has taken
-    i64 row = next_long();
-    bool whole = row >= 0;
-    Place at = whole ? claim(row, true) : claim(da + g, false);
-    int src = partner(at);
-    while (__any_sync(FULL, at.d >= 0)) {
-        const bool work = __any_sync(FULL, src >= 0);
-        if (work) fetch(src);
-        // while the copies are under way: where each lane goes next, and its partner there
-        const bool was_whole = whole;
-        Place to = at;
-        to.cur += whole ? 32 : GL;
-        // lane 0 of a group (of the warp) has the last entries: its row is done with it
-        const int lead = __shfl_sync(FULL, to.cur, whole ? 0 : lane & ~(GL - 1));
-        const bool done = at.d >= 0 && lead >= at.end;
-        const unsigned dm = __ballot_sync(FULL, done);
-        const unsigned sums = __ballot_sync(FULL, done && at.filled);
-        if (dm) {
-            if (whole) {
-                row = next_long();
-                whole = row >= 0;
-                to = whole ? claim(row, true) : claim(da + g, false);
-            } else {
-                // the finished groups take the next rows, in group order
-                const unsigned gm = dm & 0x11111111u;
-                if (done) to = claim(next + __popc(gm & ((1u << (GL * g)) - 1u)), false);
-                next += __popc(gm);
-            }
-        }
-        const int to_src = partner(to);
-        if (work) {
-            double tx = 0.0, ty = 0.0, hs = 0.0, hd = 1.0;
-            if (src >= 0) {
-                const double2 c = reinterpret_cast<const double2*>(src_center)[src];
-                const double2 cd = reinterpret_cast<const double2*>(dst_center)[da + at.d];
-                tx = cd.x - c.x;
-                ty = cd.y - c.y;
-                if (MIXED) {
-                    hs = src_half[src];
-                    hd = dst_half[da + at.d];
-                }
-            }
+    walk_rows(
+        row_start, partners, n_dst, (i64)blockIdx.x * WARPS_PER_BLOCK<T> + wib,
+        (i64)gridDim.x * WARPS_PER_BLOCK<T>, fetch,
+        [&](int to_src) {
             copies_done();
             __syncwarp();
             if (packed && to_src >= 0)
                 prefetch_l2(static_cast<const char*>(source) + (size_t)to_src * (16 * WORDS<T, P>),
                             16 * W);
-            if (src >= 0)
-                translate<P, B0, B1>(stage + lane * PITCH_S, tx, ty, eps2, hs, hd, order, acc);
-        }
-        if (done && at.filled) {
-            group_sums(sums);
-            if (was_whole) {
+        },
+        [&]() { translate<P, B0, B1>(stage + lane * PITCH_S, tx, ty, eps2, hs, hd, order, acc); },
+        [&](i64 d, bool whole, unsigned mask) {
+            group_sums(mask);
+            if (whole) {
 #pragma unroll
                 for (int k = 0; k < Q; ++k) {
-                    sum[k] += __shfl_xor_sync(FULL, sum[k], 4);
-                    sum[k] += __shfl_xor_sync(FULL, sum[k], 8);
-                    sum[k] += __shfl_xor_sync(FULL, sum[k], 16);
+                    sum[k] += __shfl_xor_sync(FULL_WARP, sum[k], 4);
+                    sum[k] += __shfl_xor_sync(FULL_WARP, sum[k], 8);
+                    sum[k] += __shfl_xor_sync(FULL_WARP, sum[k], 16);
                 }
             }
-            if (!was_whole || g == 0) add_to_locals(da + at.d);
+            if (!whole || lane < ROW_GL) add_to_locals(d);
 #pragma unroll
             for (int k = 0; k < NB + NC; ++k) acc[k] = T(0);
-        }
-        __syncwarp();
-        at = to;
-        src = to_src;
-    }
+        });
 }
 
 // Records for the M2L: m~_a (FP64), or m~_a / h^|a| (FP32); zero beyond the order.

@@ -177,6 +177,12 @@ int td3_m2l_tensor(const i64* row_start, const int* entry_row, const i64* partne
                    const float2* hat, int order, const double* coeff, double unit,
                    double* local_re, double* local_im, i64* status, cudaStream_t s);
 
+// The FP64 log M2L of orders up to 20 (m2l_log_rows.cu); arguments as td3_fmm_m2l.
+int td3_m2l_log_rows(const i64* row_start, const i64* partners, i64 n_dst,
+                     const double* dst_center, const double* src_center, const double* moment_re,
+                     const double* moment_im, int order, const double* coeff, double* local_re,
+                     double* local_im, cudaStream_t s);
+
 // The Cartesian M2L of orders up to 16 from the moments themselves (cart_m2l.cu): arguments
 // as td3_cart_m2l_mixed; FP64 without `mixed` (the half-widths are then not read).
 int td3_cart_m2l_unpacked(const i64* row_start, const i64* partners, i64 n_dst,

@@ -3,7 +3,7 @@
 //                              K/fmm_m2l/fmm_m2l_cuda.cu:12-80)
 //   L2L per level             (K/fmm_downward/fmm_downward_pyccel.py:15-64)
 //
-// M2L: one warp per destination cell; the warp splits into groups of G lanes, lane l
+// M2L (orders above 20; up to 20: m2l_log_rows.cu): one warp per destination cell; the warp splits into groups of G lanes, lane l
 // of a group owning expansion coefficient l (and l + G), each group taking every
 // (32/G)-th partner; the scaled moments a'_k = a_k w^k pass through shared memory and
 // s_l = sum_k coeff[k, l] a'_k is the real matrix product of the reference.  The
@@ -369,13 +369,10 @@ extern "C" int td3_fmm_m2l(const int64_t* row_start, const int64_t* partners, in
     if (n_dst == 0) return TD3_OK;
     cudaStream_t s = td3_stream(stream);
     int w = order + 1;
-    if (w <= 8)
-        launch_m2l<8, 1>(row_start, partners, n_dst, dst_center, src_center, moment_re, moment_im,
-                         order, coeff, local_re, local_im, s);
-    else if (w <= 16)
-        launch_m2l<16, 1>(row_start, partners, n_dst, dst_center, src_center, moment_re, moment_im,
-                          order, coeff, local_re, local_im, s);
-    else if (w <= 32)
+    if (order <= 20)
+        return td3_m2l_log_rows(row_start, partners, n_dst, dst_center, src_center, moment_re,
+                                moment_im, order, coeff, local_re, local_im, s);
+    if (w <= 32)
         launch_m2l<32, 1>(row_start, partners, n_dst, dst_center, src_center, moment_re, moment_im,
                           order, coeff, local_re, local_im, s);
     else
