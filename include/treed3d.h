@@ -685,6 +685,31 @@ int td3_soften(const double* targets, int64_t m, const double* sources, const do
                double scale, double* phi, double* field, int64_t* status, void* workspace,
                size_t workspace_bytes, void* stream);
 
+/* ------------------------------------------------------------------ simulation step */
+
+/* What a simulation step's host logic asks of the state, in one read: facts (9 doubles,
+ * device) = lowest and highest x, lowest and highest y (of non-finite positions: unspecified),
+ * and the numbers of particles with a non-finite position, with a charge, fixed, differing
+ * from the last state in position, charge or fixed (last_* null: 0; a NaN differs), and beyond
+ * a wall, wall_sign (coordinate - wall_value) > 0 (n_walls <= 4, host arrays; axis 0 or 1).
+ * pos (2, n).  Stands for the array reductions of src/tree_d_3d/simulation.py:473-495, :567-581
+ * and :625-639. */
+size_t td3_sim_scan_workspace_size(void);
+int td3_sim_scan(const double* pos, const double* charge, const uint8_t* fixed, int64_t n,
+                 const double* last_pos, const double* last_charge, const uint8_t* last_fixed,
+                 int n_walls, const int* wall_axis, const double* wall_sign,
+                 const double* wall_value, double* facts, void* workspace,
+                 size_t workspace_bytes, void* stream);
+
+/* The electric half kick and the exact cyclotron drift of a step, and its second half kick
+ * with the total force (src/tree_d_3d/simulation.py:806-835); electric (2, n) = k_e q E. */
+int td3_sim_kick_drift(const double* pos, const double* vel, const double* electric,
+                       const double* charge, const double* mass, const uint8_t* fixed, int64_t n,
+                       double dt, double b_z, double* new_pos, double* new_vel, void* stream);
+int td3_sim_kick_force(const double* vel, const double* electric, const double* charge,
+                       const double* mass, const uint8_t* fixed, int64_t n, double dt,
+                       double b_z, double* new_vel, double* force, void* stream);
+
 /* ------------------------------------------------------------------ utilities */
 
 /* Stable radix sort of (key, value) uint32 pairs by the low `bits` bits of the key.

@@ -1,0 +1,108 @@
+"""The simulation step's own kernels against the same step on array operations: sizes around
+a warp and a block, with and without a magnetic field, fixed and uncharged particles, walls
+that absorb some.  Both forms do the same operations in FP64 (sines by another routine), so
+1e-13 of the largest value.  Each step is compared on the native step's own state and fields:
+the fields of a tree are not continuous in the positions (a particle changes its cell).
+"""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from conftest import relative
+
+pytestmark = pytest.mark.gpu
+
+
+def _simulation(n, b_z, kind):
+    from tree_d_3d_b200 import Quad
+    from tree_d_3d_b200.simulation import ElectrostaticSimulation
+
+    rng = np.random.default_rng(n)
+    charges, fixed = rng.choice([-1.0, 1.0], n), np.zeros(n, dtype=bool)
+    if kind == "mixed":
+        charges[::3] = 0.0
+        fixed[1::4] = True
+    return ElectrostaticSimulation(
+        positions=rng.uniform(-0.9, 0.9, (2, n)), velocities=rng.normal(size=(2, n)),
+        charges=charges, masses=rng.uniform(0.5, 2, n), fixed=fixed, bounds=Quad(0, 0, 1),
+        k_e=1e-2, softening=1e-2, dt=0.05, B_z=b_z, kernel="log" if kind == "log" else "coulomb",
+        absorbing_walls={"x_max": 0.95, "y_min": -0.95} if kind != "free" else {"x_min": -50.0})
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 257, 1500])
+@pytest.mark.parametrize("b_z,kind", [(0.0, "free"), (1.5, "free"), (1.5, "mixed"), (0.7, "log")])
+def test_native_step_matches_the_array_step(n, b_z, kind):
+    from tree_d_3d_b200.simulation import ElectrostaticSimulation
+
+    from tree_d_3d_b200.simulation import _drift
+
+    sim = _simulation(n, b_z, kind)
+    assert sim._native()
+    for _ in range(3):
+        sim.compute_fields(include_fixed=False, potential=False)
+        pos, vel, electric = sim.positions, sim.velocities, sim._electric
+        q, m, mobile = sim.charges, sim.masses, (~sim.fixed).double()
+        sim.step()
+        vel = vel + 0.5 * sim.dt * electric / m * mobile
+        pos, vel = _drift(pos, vel, q, m, sim.B_z, sim.dt, mobile)
+        inside = torch.ones_like(q, dtype=torch.bool)
+        for _, axis, sign, value in sim._walls:
+            inside &= ~(sign * (pos[axis] - value) > 0)
+        assert sim.num_particles == int(inside.sum())
+        if not sim.num_particles:
+            break
+        pos, vel, q, m, mobile = pos[:, inside], vel[:, inside], q[inside], m[inside], mobile[inside]
+        vel = vel + 0.5 * sim.dt * sim._electric / m * mobile
+        forces = sim._electric + q * sim.B_z * torch.stack((vel[1], -vel[0]))
+        for a, b in ((sim.positions, pos), (sim.velocities, vel), (sim.forces, forces)):
+            assert relative(a.cpu().numpy(), b.cpu().numpy()) < 1e-13
+
+
+def test_step_sees_a_state_changed_in_place_and_refuses_non_finite_positions():
+    sim = _simulation(100, 1.0, "free")
+    sim.compute_fields()
+    before = sim._electric.clone()
+    sim.compute_fields()
+    assert torch.equal(sim._electric, before)
+    sim.charges[3] *= 2
+    sim.compute_fields()
+    assert not torch.equal(sim._electric, before)
+    sim.positions[0, 5] = float("nan")
+    with pytest.raises(ValueError, match="finite"):
+        sim.step()
+
+
+def test_velocities_that_autograd_follows_step_on_array_operations():
+    sim = _simulation(50, 1.0, "free")
+    sim.velocities.requires_grad_(True)
+    assert not sim._native()
+    v = sim.velocities
+    sim.step()
+    sim.velocities.sum().backward()
+    assert v.grad is not None
+
+
+def test_pair_sum_logarithm_and_reciprocal():
+    """direct_field of the log kernel at single distances: phi = -ln r^2 and E = 2 / r to a few
+    units in the last place at every magnitude (the table's intervals, both sides of r = 1,
+    where ln r^2 must keep its relative accuracy, and beyond the short form's range)."""
+    from tree_d_3d_b200 import direct_field
+
+    rng = np.random.default_rng(0)
+    near = 1 + np.concatenate([s * 2.0 ** -np.arange(1.0, 50.0) for s in (1, -1)])
+    r = np.concatenate([np.exp(rng.uniform(-300, 300, 20000)), rng.uniform(0.5, 2, 20000), near,
+                        2.0 ** np.arange(-530, 505.0), [1.0, 1e-155, 1e-160, 1e153, 1e154]])
+    phi, field = direct_field(torch.tensor(np.stack((r, 0 * r)), device="cuda"),
+                              torch.zeros((2, 1), device="cuda", dtype=torch.float64),
+                              torch.ones(1, device="cuda", dtype=torch.float64), kernel="log")
+    r2 = r * r
+    with np.errstate(over="ignore"):
+        want, inverse = -np.log(r2), 2 / r2 * r
+    assert not field[1].cpu().numpy()[np.isfinite(inverse)].any()
+    for got, ref in ((phi.cpu().numpy(), want), (field[0].cpu().numpy(), inverse)):
+        finite = np.isfinite(ref)  # 2 / r^2 of a denormal r^2 is infinite
+        assert np.array_equal(got[~finite], ref[~finite])
+        assert np.all(np.abs(got[finite] - ref[finite]) <= 4 * np.spacing(np.abs(ref[finite])))

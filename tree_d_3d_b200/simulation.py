@@ -101,15 +101,25 @@ def _drift(pos, vel, charges, masses, b_z, dt, mobile):
     return pos, vel
 
 
-def _expanded_root(bounds: Quad, points: torch.Tensor) -> Quad:
+class _Facts:
+    """The state in numbers (td3_sim_scan): one host read for the questions that a step's
+    host logic asks."""
+
+    def __init__(self, values) -> None:
+        self.low, self.high = [values[0], values[2]], [values[1], values[3]]
+        self.not_finite, self.charged, self.fixed, self.changed, self.outside = (
+            int(v) for v in values[4:9])
+
+
+def _expanded_root(bounds: Quad, points: torch.Tensor, facts: _Facts | None = None) -> Quad:
     """The root enlarged to hold ``points`` (simulation.py:625-639)."""
     if not points.shape[1]:
         return bounds
-    if not bool(torch.isfinite(points).all()):
+    if facts.not_finite if facts is not None else not bool(torch.isfinite(points).all()):
         raise ValueError("Particle positions must be finite; reduce dt")
     b = bounds
-    lo = points.amin(dim=1).tolist()
-    hi = points.amax(dim=1).tolist()
+    lo = facts.low if facts is not None else points.amin(dim=1).tolist()
+    hi = facts.high if facts is not None else points.amax(dim=1).tolist()
     lo = [min(lo[0], b.xmid - b.half), min(lo[1], b.ymid - b.half)]
     hi = [max(hi[0], b.xmid + b.half), max(hi[1], b.ymid + b.half)]
     if (lo[0] < b.xmid - b.half or lo[1] < b.ymid - b.half or hi[0] > b.xmid + b.half
@@ -212,13 +222,51 @@ class ElectrostaticSimulation:
             which = torch.where(deeper, torch.full_like(which, k), which)
         return which >= 0, which
 
-    def _absorb(self) -> None:
-        """simulation.py:508-565: remove and record the particles beyond a wall."""
-        if not self._walls:
-            return
+    def _native(self) -> bool:
+        """Whether the state's arrays are as the step's own kernels take them (as the
+        constructor makes them, and nothing that autograd follows); otherwise a step runs
+        on array operations."""
+        n, grad = self.num_particles, torch.is_grad_enabled()
+        for array, shape in ((self.positions, (2, n)), (self.velocities, (2, n)),
+                             (self._electric, (2, n)), (self.charges, (n,)),
+                             (self.masses, (n,)), (self.fixed, (n,))):
+            dtype = torch.bool if array is self.fixed else torch.float64
+            if (type(array) is not torch.Tensor or array.dtype != dtype or not array.is_cuda
+                    or tuple(array.shape) != shape or not array.is_contiguous()
+                    or (grad and array.requires_grad)):
+                return False
+        return True
+
+    def _scan(self) -> _Facts | None:
+        """The state's facts (None where its arrays are not the kernels' kind)."""
+        if not self._native():
+            return None
+        n, dev = self.num_particles, self.positions.device
+        last = [0, 0, 0]
+        state = self._field_state
+        if state is not None and state[0].shape == self.positions.shape:
+            if [t.dtype for t in state[:3]] != [torch.float64, torch.float64, torch.bool]:
+                return None  # fields of other arrays: compared as arrays
+            last = [t.data_ptr() for t in state[:3]]
+        axis = np.array([w[1] for w in self._walls], dtype=np.int32)
+        sign = np.array([w[2] for w in self._walls], dtype=np.float64)
+        value = np.array([w[3] for w in self._walls], dtype=np.float64)
+        out = torch.empty(9, dtype=torch.float64, device=dev)
+        ws = _lib.workspace(_lib.query("td3_sim_scan_workspace_size"), dev)
+        _lib.call("td3_sim_scan", self.positions.data_ptr(), self.charges.data_ptr(),
+                  self.fixed.data_ptr(), n, *last, len(self._walls), axis.ctypes.data,
+                  sign.ctypes.data, value.ctypes.data, out.data_ptr(), ws.data_ptr(), ws.numel(),
+                  _lib.stream(dev))
+        return _Facts(out.tolist())
+
+    def _absorb(self, facts: _Facts | None = None) -> bool:
+        """simulation.py:508-565: remove and record the particles beyond a wall; whether
+        there were any."""
+        if not self._walls or (facts is not None and not facts.outside):
+            return False
         outside, which = self._outside()
         if not bool(outside.any()):
-            return
+            return False
         names = [self._walls[int(k)][0] for k in which[outside].tolist()]
         self.absorbed.record(time=self.current_time + self.dt, walls=names,
                              positions=self.positions[:, outside],
@@ -231,13 +279,14 @@ class ElectrostaticSimulation:
             setattr(self, name, getattr(self, name)[keep].contiguous())
         self._field_state = None
         self._tree = None
+        return True
 
     # ------------------------------------------------------------------ fields
-    def _resolve_method(self) -> str:
+    def _resolve_method(self, facts: _Facts | None = None) -> str:
         """simulation.py:567-581 (the Coulomb FMM runs on the GPU here)."""
         if self.method != "auto":
             return self.method
-        charged = int(torch.count_nonzero(self.charges))
+        charged = facts.charged if facts is not None else int(torch.count_nonzero(self.charges))
         if self.theta == 0 or charged <= self.direct_threshold:
             return "direct"
         return "fmm" if self.theta < 1 else "tree"
@@ -247,11 +296,14 @@ class ElectrostaticSimulation:
                 self.leaf_capacity, self.max_depth, self.kernel, self.order,
                 self.reference_radius, self.precision)
 
-    def _fields_current(self) -> bool:
+    def _fields_current(self, facts: _Facts | None = None) -> bool:
         state = self._field_state
         if state is None:
             return False
         pos, charge, fixed, params = state
+        if facts is not None:
+            return (params == self._parameters() and pos.shape == self.positions.shape
+                    and not facts.changed)
         return (params == self._parameters() and torch.equal(pos, self.positions)
                 and torch.equal(charge, self.charges) and torch.equal(fixed, self.fixed))
 
@@ -273,25 +325,33 @@ class ElectrostaticSimulation:
     def compute_fields(self, include_fixed: bool = True, potential: bool = True):
         """Electric force and potential on every particle, reused while the state is
         unchanged (simulation.py:704-798).  Returns the tree used (None: direct)."""
+        return self._compute_fields(include_fixed, potential, self._scan())
+
+    def _compute_fields(self, include_fixed: bool, potential: bool, facts: _Facts | None):
         want_potential = potential or self.kernel != "log"
         if want_potential and not self._potential_done and self._field_state is not None:
             self._field_state = None
-        if self._fields_current():
+        if self._fields_current(facts):
             return self._tree
         n = self.num_particles
-        self.bounds = _expanded_root(self.bounds, self.positions)
-        method = self._resolve_method()
+        self.bounds = _expanded_root(self.bounds, self.positions, facts)
+        method = self._resolve_method(facts)
         self._potential_done = want_potential or method == "direct"
         self._tree = None
         phi = torch.zeros(n, dtype=torch.float64, device=self.positions.device)
         field = torch.zeros_like(self.positions)
-        charged = self.charges != 0
-        if self.k_e != 0 and n and bool(charged.any()):
+        if self.k_e != 0 and n and (facts.charged if facts is not None
+                                    else bool((self.charges != 0).any())):
             if method == "fmm":
                 self._tree = self._make_tree(method)
                 phi, field = self._tree.fmm(theta=self.theta, softening=self.softening,
                                             potential=self._potential_done)
+            elif (method == "direct" and facts is not None and facts.charged == n
+                  and (include_fixed or not facts.fixed)):  # every particle is a target
+                phi, field = _direct(self.positions, torch.arange(n, device=self.charges.device),
+                                     self.positions, self.charges, self.softening, self.kernel)
             else:
+                charged = self.charges != 0
                 targets = torch.nonzero(charged & (include_fixed | ~self.fixed)).flatten()
                 tpos = self.positions[:, targets].contiguous()
                 if method == "tree":
@@ -319,18 +379,42 @@ class ElectrostaticSimulation:
         (simulation.py:800-835).  Returns the tree of the end-of-step forces."""
         self.dt = _finite("dt", self.dt if dt is None else dt, positive=True)
         self.compute_fields(include_fixed=False, potential=False)
-        mobile = (~self.fixed).to(torch.float64)
-        self.velocities = self.velocities + 0.5 * self.dt * self._electric / self.masses * mobile
-        self.positions, self.velocities = _drift(self.positions, self.velocities, self.charges,
-                                                 self.masses, self.B_z, self.dt, mobile)
-        self._absorb()
-        tree = self.compute_fields(include_fixed=False, potential=False)
-        mobile = (~self.fixed).to(torch.float64)
-        self.velocities = self.velocities + 0.5 * self.dt * self._electric / self.masses * mobile
-        vx, vy = self.velocities
-        self.forces = self._electric + self.charges * self.B_z * torch.stack((vy, -vx))
+        if self._native():
+            tree = self._native_step()
+        else:
+            mobile = (~self.fixed).to(torch.float64)
+            self.velocities = self.velocities + 0.5 * self.dt * self._electric / self.masses * mobile
+            self.positions, self.velocities = _drift(self.positions, self.velocities, self.charges,
+                                                     self.masses, self.B_z, self.dt, mobile)
+            self._absorb()
+            tree = self.compute_fields(include_fixed=False, potential=False)
+            mobile = (~self.fixed).to(torch.float64)
+            self.velocities = self.velocities + 0.5 * self.dt * self._electric / self.masses * mobile
+            vx, vy = self.velocities
+            self.forces = self._electric + self.charges * self.B_z * torch.stack((vy, -vx))
         self.current_time += self.dt
         self.iteration += 1
+        return tree
+
+    def _native_step(self):
+        """The rest of a step after its first fields, the arrays' parts in the library's
+        kernels (one read of the state's facts for the walls and the next fields)."""
+        n, stream = self.num_particles, _lib.stream(self.positions.device)
+        pos, vel = torch.empty_like(self.positions), torch.empty_like(self.velocities)
+        _lib.call("td3_sim_kick_drift", self.positions.data_ptr(), self.velocities.data_ptr(),
+                  self._electric.data_ptr(), self.charges.data_ptr(), self.masses.data_ptr(),
+                  self.fixed.data_ptr(), n, self.dt, self.B_z, pos.data_ptr(), vel.data_ptr(),
+                  stream)
+        self.positions, self.velocities = pos, vel
+        facts = self._scan()
+        if self._absorb(facts):
+            facts = self._scan()
+        tree = self._compute_fields(False, False, facts)
+        vel, forces = torch.empty_like(self.velocities), torch.empty_like(self.positions)
+        _lib.call("td3_sim_kick_force", self.velocities.data_ptr(), self._electric.data_ptr(),
+                  self.charges.data_ptr(), self.masses.data_ptr(), self.fixed.data_ptr(),
+                  self.num_particles, self.dt, self.B_z, vel.data_ptr(), forces.data_ptr(), stream)
+        self.velocities, self.forces = vel, forces
         return tree
 
     # ------------------------------------------------------------------ diagnostics
