@@ -116,3 +116,18 @@ def test_cartesian_records_reject_other_orders():
     assert lib.td3_cart_record_bytes(17, 0) == _lib.EINVAL
     assert lib.td3_pack_cart_sources(1, 17, 0, 0, 0, 0, 0) == _lib.EINVAL
     assert lib.td3_cart_m2l_rows(0, 0, 1, 0, 0, 0, 0, 0, 17, 0.0, 0, 0, 0) == _lib.EINVAL
+
+
+@pytest.mark.parametrize("mixed", [0, 1])
+@pytest.mark.parametrize("order", [0, 2, 6, 10, 14])
+def test_unpacked_moments_do_not_read_what_shared_memory_held(order, mixed):
+    """Orders below their template's: moments above the order count as zero, whatever the
+    launch before (NaN moments of the template's order) left in shared memory."""
+    c = _case(order, 1e-3, order)
+    full = 4 if order <= 4 else 8 if order <= 8 else 12 if order <= 12 else 16
+    nans = _case(full, 1e-3, order)
+    nans["moments"] = np.full_like(nans["moments"], np.nan)
+    for _ in range(5):
+        assert np.isnan(_run(nans, full, mixed, True)).any()
+        got = _run(c, order, mixed, False)
+        assert np.isfinite(got).all()

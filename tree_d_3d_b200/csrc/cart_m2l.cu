@@ -392,9 +392,11 @@ k_m2l_cart_rows(const i64* __restrict__ row_start, const i64* __restrict__ partn
                 const int s = __shfl_sync(FULL_WARP, src, p);
                 if (s < 0) continue;
                 const double inv_h = MIXED ? 1.0 / src_half[s] : 1.0;
-                for (int a = lane; a < n_coef && a < tri(NA + 1); a += 32) {
+                // zeros above the order, as in a record: products() multiplies degree order + 1
+                // by 0, and what shared memory held may be a NaN
+                for (int a = lane; a < tri(NA + 1); a += 32) {
                     const int na = degree_of(a);
-                    double v = mom[(size_t)s * n_coef + a] * C.inv_fact2[a];
+                    double v = a < n_coef ? mom[(size_t)s * n_coef + a] * C.inv_fact2[a] : 0.0;
                     if (na & 1) v = -v;
                     if (MIXED)
                         for (int k = 0; k < na; ++k) v *= inv_h;
