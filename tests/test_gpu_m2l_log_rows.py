@@ -51,3 +51,18 @@ def test_log_m2l_rows_match_the_oracle(oracle, order, copies):
         if want is want_im:  # Im b_0 never enters the field (its branch is not fixed)
             got, want = got[:, 1:], want[:, 1:]
         assert np.all(np.max(np.abs(got - want), 0) <= 1e-12 * np.max(np.abs(want), 0))
+
+
+@pytest.mark.parametrize("order", [5, 9, 11])
+def test_powers_above_the_order_may_overflow(order):
+    """Cells so small that 1 / t^k overflows above the order only: lengths of 2^-k and the
+    field of 2^k are exact, so the scaled solve agrees to the rounding of its logarithms."""
+    from tree_d_3d_b200 import FlatQuadtree, Quad
+
+    rng = np.random.default_rng(order)
+    pos, q = rng.uniform(-1, 1, (2, 4000)), rng.normal(size=4000)
+    scale = 2.0 ** -{5: 133, 9: 96, 11: 82}[order]
+    _, want = FlatQuadtree(pos, q, Quad(0, 0, 1), kernel="log", order=order).fmm()
+    _, got = FlatQuadtree(scale * pos, q, Quad(0, 0, scale), kernel="log", order=order).fmm()
+    assert np.isfinite(got).all()
+    assert np.max(np.abs(got * scale - want)) < 1e-12 * np.max(np.abs(want))

@@ -87,9 +87,11 @@ k_m2l_log_rows(const i64* __restrict__ row_start, const i64* __restrict__ partne
         double pr = 1.0, pi = 0.0;
 #pragma unroll
         for (int k = 0; k < W; ++k) {
-            const double xr = k < w ? own[k] : 0.0, xi = k < w ? own[W + k] : 0.0;
-            ar[k] = xr * pr - xi * pi;
-            ai[k] = xr * pi + xi * pr;
+            const double xr = own[k], xi = own[W + k];
+            // above the order: zero by selection (the place is not written, and w^k may be
+            // infinite where w^order is not)
+            ar[k] = k < w ? xr * pr - xi * pi : 0.0;
+            ai[k] = k < w ? xr * pi + xi * pr : 0.0;
             const double nr = pr * wr - pi * wi;
             pi = pr * wi + pi * wr;
             pr = nr;
