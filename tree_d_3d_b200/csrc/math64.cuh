@@ -1,5 +1,5 @@
-// FP64 logarithm and reciprocal of the pair sums, without the library functions' branches.
-// Both for arguments between 2^-1007 and 2^992 (in_range64; callers take the library's
+// FP64 logarithm, reciprocal and reciprocal square root of the pair sums, without the library
+// functions' branches.  All for arguments between 2^-1007 and 2^992 (in_range64; callers take the library's
 // functions elsewhere: zeros, denormals, infinities and NaN keep their results).
 //
 // ln x by a table and a short polynomial (P. T. P. Tang, Table-driven implementation of the
@@ -9,8 +9,9 @@
 // |r| <= 2^-9 (2^-8 at 1): ln x = k ln 2 - ln c + ln(1 + r), the last by its series to r^7 / 7
 // (the next term is below 2^-67).  12 FP64 operations and one 16-byte read.
 //
-// 1 / x from the hardware's approximation y (about 2^-20) by one step of third order,
-// y (1 + e + e^2), e = 1 - x y: an error of e^3.
+// 1 / x and x^(-1/2) from the hardware's approximations y (about 2^-20) by one step of third
+// order: y (1 + e + e^2) with e = 1 - x y, and y (1 + e / 2 + 3 e^2 / 8) with e = 1 - x y^2; the
+// errors are of the order of e^3.
 #pragma once
 
 #include "common.cuh"
@@ -53,4 +54,17 @@ __device__ __forceinline__ double reciprocal64(double x) {
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     const double e = fma(-x, y, 1.0);
     return fma(y, fma(e, e, e), y);
+}
+
+__device__ __forceinline__ double rsqrt64(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(y, e * fma(e, 0.375, 0.5), y);
+}
+
+// The same for every argument.
+__device__ __forceinline__ double rsqrt_any(double x) { return in_range64(x) ? rsqrt64(x) : rsqrt(x); }
+__device__ __forceinline__ double reciprocal_any(double x) {
+    return in_range64(x) ? reciprocal64(x) : 1.0 / x;
 }
