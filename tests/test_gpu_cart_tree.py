@@ -78,3 +78,18 @@ def test_cartesian_l2l_matches_the_oracle(oracle, order, capacity):
         for n in range(order + 1):
             a, b = got[rows][:, degree == n], want[rows][:, degree == n]
             assert np.max(np.abs(a - b)) <= 1e-12 * np.max(np.abs(b))
+
+
+@pytest.mark.parametrize("order,capacity", [(16, 1), (31, 8), (32, 9), (33, 40), (63, 7), (64, 17)])
+def test_log_moments_of_high_orders_equal_the_oracle(oracle, order, capacity):
+    """Orders above 15 (a warp per node, 8 particles at a time): the oracle's bits."""
+    from tree_d_3d_b200 import FlatQuadtree, Quad
+
+    rng = np.random.default_rng(order)
+    pos = np.concatenate([rng.uniform(-1, 1, (2, 500)), rng.normal(0.3, 0.01, (2, 500))], 1)
+    q = rng.normal(size=1000)
+    ref = oracle.OracleTree(pos, q, (0, 0, 1), kernel="log", order=order, leaf_capacity=capacity)
+    tree = FlatQuadtree(pos, q, Quad(0, 0, 1), kernel="log", order=order, leaf_capacity=capacity)
+    for name in ("node_qabs", "moment_re", "moment_im"):
+        got = getattr(tree, name)
+        np.testing.assert_array_equal(got.cpu().numpy(), getattr(ref, name))

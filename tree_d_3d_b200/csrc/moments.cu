@@ -60,79 +60,114 @@ __global__ void k_coulomb_moments(i64 lo, i64 hi, const double* __restrict__ spo
     node_s[3 * node + 2] = syy;
 }
 
-// One thread per (node, n), n = 0..order.  sdip (2, n_particles; may be null) adds
-// point dipoles e = (ex, ey) at the particles: a_n -= n e (z - c)^(n - 1), the moments
-// of the adjoint (transposed) FMM pass, whose sources are monopoles and dipoles.
-__global__ void k_log_moments(i64 lo, i64 hi, int order, const double* __restrict__ spos,
-                              const double* __restrict__ scharge, i64 n_particles,
-                              const double* __restrict__ node_center,
-                              const i64* __restrict__ node_start, const i64* __restrict__ node_end,
-                              const i64* __restrict__ node_child,
-                              const double* __restrict__ binomial, int bsize, double* node_qabs,
-                              double* moment_re, double* moment_im,
-                              const double* __restrict__ sdip) {
-    i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    int w = order + 1;
-    i64 node = lo + t / w;
-    int n = (int)(t % w);
+// Log moments of orders above 15, level by level, a warp per node.  The powers that every
+// coefficient needs (a particle's q z^n, and z^n with dipoles; a child's shift) are one serial
+// chain each: a lane forms a particle's (a child's) once in shared memory, where lane n sums
+// its coefficients in particle (child) order.  The latency of those chains and of a level's
+// launch bounds it.
+constexpr int LOG_MOM_WARPS = 2;
+constexpr int LOG_MOM_SLOTS = 8;  // particles at a time, or 4 shifts and 4 children's moments
+constexpr int LOG_MOM_PER_LANE = (TD3_MAX_ORDER + 32) / 32;
+
+__global__ void __launch_bounds__(32 * LOG_MOM_WARPS)
+k_log_moments(i64 lo, i64 hi, int order, const double* __restrict__ spos,
+              const double* __restrict__ scharge, i64 n_particles,
+              const double* __restrict__ node_center, const i64* __restrict__ node_start,
+              const i64* __restrict__ node_end, const i64* __restrict__ node_child,
+              const double* __restrict__ binomial, int bsize, double* node_qabs,
+              double* moment_re, double* moment_im, const double* __restrict__ sdip) {
+    extern __shared__ double2 log_mom_smem[];
+    td3_chain_wait();
+    td3_chain_release();
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const i64 node = lo + (i64)blockIdx.x * LOG_MOM_WARPS + wib;
     if (node >= hi) return;
-    double xmid = node_center[2 * node], ymid = node_center[2 * node + 1];
-    double acc_re = 0.0, acc_im = 0.0, qabs = 0.0;
-    i64 first = node_child[node];
+    const int w = order + 1, pitch = w | 1;  // odd: the lanes' writes hit distinct banks
+    double2* slot = log_mom_smem + (size_t)wib * (sdip ? 2 : 1) * LOG_MOM_SLOTS * pitch;
+    const double xmid = node_center[2 * node], ymid = node_center[2 * node + 1];
+    double acc_re[LOG_MOM_PER_LANE], acc_im[LOG_MOM_PER_LANE], qabs = 0.0;
+#pragma unroll
+    for (int c = 0; c < LOG_MOM_PER_LANE; ++c) acc_re[c] = acc_im[c] = 0.0;
+    const i64 first = node_child[node];
     if (first < 0) {
-        for (i64 k = node_start[node]; k < node_end[node]; ++k) {
-            double q = scharge[k];
-            qabs += fabs(q);
-            double dx = spos[k] - xmid, dy = spos[n_particles + k] - ymid;
-            double pr = q, pi = 0.0;
-            for (int m = 0; m < n; ++m) {
-                double next_re = pr * dx - pi * dy;
-                pi = pr * dy + pi * dx;
-                pr = next_re;
-            }
-            acc_re += pr;
-            acc_im += pi;
-            if (sdip && n > 0) {
-                // - n e (z - c)^(n-1)
-                double er = sdip[k], ei = sdip[n_particles + k];
-                double zr = 1.0, zi = 0.0;
-                for (int m = 0; m < n - 1; ++m) {
-                    double nr = zr * dx - zi * dy;
-                    zi = zr * dy + zi * dx;
-                    zr = nr;
+        const i64 end = node_end[node];
+        for (i64 k0 = node_start[node]; k0 < end; k0 += LOG_MOM_SLOTS) {
+            const int count = end - k0 < LOG_MOM_SLOTS ? (int)(end - k0) : LOG_MOM_SLOTS;
+            const int p = lane % LOG_MOM_SLOTS, kind = lane / LOG_MOM_SLOTS;
+            __syncwarp();
+            if (p < count && kind < (sdip ? 2 : 1)) {
+                const double dx = spos[k0 + p] - xmid, dy = spos[n_particles + k0 + p] - ymid;
+                double2 z = make_double2(kind ? 1.0 : scharge[k0 + p], 0.0);
+                for (int n = 0; n < w; ++n) {
+                    slot[lane * pitch + n] = z;
+                    z = make_double2(z.x * dx - z.y * dy, z.x * dy + z.y * dx);
                 }
-                acc_re -= n * (er * zr - ei * zi);
-                acc_im -= n * (er * zi + ei * zr);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < LOG_MOM_PER_LANE; ++c) {
+                const int n = lane + 32 * c;
+                if (n >= w) continue;
+                for (int j = 0; j < count; ++j) {
+                    const double2 v = slot[j * pitch + n];
+                    if (n == 0) qabs += fabs(v.x);
+                    acc_re[c] += v.x;
+                    acc_im[c] += v.y;
+                    if (sdip && n > 0) {
+                        // - n e (z - c)^(n-1)
+                        const double er = sdip[k0 + j], ei = sdip[n_particles + k0 + j];
+                        const double2 z = slot[(LOG_MOM_SLOTS + j) * pitch + n - 1];
+                        acc_re[c] -= n * (er * z.x - ei * z.y);
+                        acc_im[c] -= n * (er * z.y + ei * z.x);
+                    }
+                }
             }
         }
     } else {
-        double sh_re[TD3_MAX_ORDER + 1], sh_im[TD3_MAX_ORDER + 1];
-        for (i64 child = first; child < first + 4; ++child) {
-            qabs += node_qabs[child];
-            if (node_end[child] == node_start[child]) continue;
-            double s_re = node_center[2 * child] - xmid;
-            double s_im = node_center[2 * child + 1] - ymid;
-            sh_re[0] = 1.0;
-            sh_im[0] = 0.0;
-            for (int k = 1; k <= n; ++k) {
-                sh_re[k] = sh_re[k - 1] * s_re - sh_im[k - 1] * s_im;
-                sh_im[k] = sh_re[k - 1] * s_im + sh_im[k - 1] * s_re;
+        if (lane < 4) {
+            const double s_re = node_center[2 * (first + lane)] - xmid;
+            const double s_im = node_center[2 * (first + lane) + 1] - ymid;
+            double2 z = make_double2(1.0, 0.0);
+            for (int n = 0; n < w; ++n) {
+                slot[lane * pitch + n] = z;
+                z = make_double2(z.x * s_re - z.y * s_im, z.x * s_im + z.y * s_re);
             }
-            double c_re = 0.0, c_im = 0.0;
-            for (int m = 0; m <= n; ++m) {
-                double c = binomial[n * bsize + m];
-                double a_re = moment_re[child * w + m] * c;
-                double a_im = moment_im[child * w + m] * c;
-                c_re += a_re * sh_re[n - m] - a_im * sh_im[n - m];
-                c_im += a_re * sh_im[n - m] + a_im * sh_re[n - m];
+        }
+        for (int j = 0; j < 4; ++j)
+            for (int m = lane; m < w; m += 32)
+                slot[(4 + j) * pitch + m] = make_double2(moment_re[(first + j) * w + m],
+                                                         moment_im[(first + j) * w + m]);
+        __syncwarp();
+        for (int j = 0; j < 4; ++j) {
+            qabs += node_qabs[first + j];
+            if (node_end[first + j] == node_start[first + j]) continue;
+            const double2 *shift = slot + j * pitch, *moment = slot + (4 + j) * pitch;
+#pragma unroll
+            for (int c = 0; c < LOG_MOM_PER_LANE; ++c) {
+                const int n = lane + 32 * c;
+                if (n >= w) continue;
+                double c_re = 0.0, c_im = 0.0;
+#pragma unroll 4
+                for (int m = 0; m <= n; ++m) {
+                    const double b = binomial[n * bsize + m];
+                    const double a_re = moment[m].x * b, a_im = moment[m].y * b;
+                    const double2 sh = shift[n - m];
+                    c_re += a_re * sh.x - a_im * sh.y;
+                    c_im += a_re * sh.y + a_im * sh.x;
+                }
+                acc_re[c] += c_re;
+                acc_im[c] += c_im;
             }
-            acc_re += c_re;
-            acc_im += c_im;
         }
     }
-    moment_re[node * w + n] = acc_re;
-    moment_im[node * w + n] = acc_im;
-    if (n == 0) node_qabs[node] = qabs;
+#pragma unroll
+    for (int c = 0; c < LOG_MOM_PER_LANE; ++c) {
+        const int n = lane + 32 * c;
+        if (n >= w) continue;
+        moment_re[node * w + n] = acc_re[c];
+        moment_im[node * w + n] = acc_im[c];
+    }
+    if (lane == 0) node_qabs[node] = qabs;
 }
 
 
@@ -403,7 +438,7 @@ k_log_moments_tree(i64 count, int order, const double* __restrict__ spos,
 
 // Moments of every node.  Orders up to 15: every leaf in one launch (leaves depend on
 // nothing), then the internal nodes level by level, deepest first, a thread per (node,
-// child); higher orders: thread per (node, coefficient), level by level.
+// child); higher orders: a warp per node, level by level.
 int launch_log_moments(const int64_t* levels, int64_t n_levels, int order, const double* spos,
                        const double* scharge, int64_t n, const double* center, const i64* start,
                        const i64* end, const i64* child, const double* binomial, int bsize,
@@ -446,9 +481,16 @@ int launch_log_moments(const int64_t* levels, int64_t n_levels, int order, const
         for (i64 level = n_levels - 1; level >= 0; --level) {
             i64 lo = levels[level], hi = levels[level + 1];
             if (hi <= lo) continue;
-            k_log_moments<<<td3_blocks((hi - lo) * (order + 1), MOM_THREADS), MOM_THREADS, 0,
-                            s>>>(lo, hi, order, spos, scharge, n, center, start, end, child,
-                                 binomial, bsize, qabs, mre, mim, sdip);
+            const size_t smem = sizeof(double2) * LOG_MOM_WARPS * LOG_MOM_SLOTS * (sdip ? 2 : 1) *
+                                ((order + 1) | 1);
+            if (smem > 48 * 1024)
+                TD3_TRY(cudaFuncSetAttribute(k_log_moments, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)smem));
+            TD3_TRY(td3_launch_chained(k_log_moments,
+                                       (unsigned)((hi - lo + LOG_MOM_WARPS - 1) / LOG_MOM_WARPS),
+                                       32 * LOG_MOM_WARPS, smem, s, lo, hi, order, spos, scharge, n,
+                                       center, start, end, child, binomial, bsize, qabs, mre, mim,
+                                       sdip));
         }
     }
     TD3_CHECK_LAUNCH();
