@@ -64,7 +64,8 @@ __global__ void k_coulomb_moments(i64 lo, i64 hi, const double* __restrict__ spo
 // coefficient needs (a particle's q z^n, and z^n with dipoles; a child's shift) are one serial
 // chain each: a lane forms a particle's (a child's) once in shared memory, where lane n sums
 // its coefficients in particle (child) order.  The latency of those chains and of a level's
-// launch bounds it.
+// launch bounds it.  With a thread per coefficient, each forming every power it needed in local
+// memory, a product of 48,000 panels (order 32) took 863 us; this way 783 us.
 constexpr int LOG_MOM_WARPS = 2;
 constexpr int LOG_MOM_SLOTS = 8;  // particles at a time, or 4 shifts and 4 children's moments
 constexpr int LOG_MOM_PER_LANE = (TD3_MAX_ORDER + 32) / 32;
