@@ -178,3 +178,18 @@ def test_panel_tree_root_is_the_widened_bounding_square():
     assert (q.xmid, q.ymid) == (0.125, -0.04999999999999999)
     assert q.half == 0.5 * 1.25 * (1 + 1e-9) + 1e-300
     assert (FMM_AT_THETA, FMM_AT_RATIO, WALK_THETA) == (0.5, 8, 0.7)
+
+
+def test_short_traversal_workspaces_are_refused():
+    """A workspace too short for any one of the traversal's buffers is refused before any CUDA
+    call, also where a later, smaller buffer would still fit in what is left."""
+    from tree_d_3d_b200 import _lib
+
+    lib = _lib.lib()
+    sizes = np.zeros(4, dtype=np.int64)
+    for frontier, nodes in ((100_000, 9), (3_000, 9), (3_000, 2_000)):
+        need = lib.td3_fmm_traverse_workspace_size(frontier, nodes)
+        for short in (256, need // 8, need // 3, need // 2, need - 2048):
+            rc = lib.td3_fmm_traverse(0, 0, 0, 0, 0, nodes, 0.5, 0, 0, 0, 0, frontier,
+                                      sizes.ctypes.data, 0, int(short), 0)
+            assert rc == _lib.EWORKSPACE, (frontier, nodes, short)

@@ -76,7 +76,10 @@ struct Workspace {
     template <typename T>
     __host__ T* take(i64 count) {
         size_t bytes = ((size_t)(count > 0 ? count : 1) * sizeof(T) + 255) & ~(size_t)255;
-        if (used + bytes > size) return nullptr;
+        if (used + bytes > size) {
+            used = size;  // the later ones fail too: a caller checks its last buffer only
+            return nullptr;
+        }
         T* out = reinterpret_cast<T*>(base + used);
         used += bytes;
         return out;
