@@ -75,6 +75,34 @@ def test_step_sees_a_state_changed_in_place_and_refuses_non_finite_positions():
         sim.step()
 
 
+def test_fields_of_a_transposed_state_are_not_taken_for_another_of_the_same_memory():
+    """The saved state is compared by its values: positions given as a.T and then, of the same
+    numbers in memory, as a.reshape(2, n) are two states."""
+    from tree_d_3d_b200 import Quad
+    from tree_d_3d_b200.simulation import ElectrostaticSimulation
+
+    n = 500
+    rng = np.random.default_rng(7)
+    a = torch.tensor(rng.uniform(-0.9, 0.9, (n, 2)), device="cuda")
+
+    def simulation(positions):
+        return ElectrostaticSimulation(positions=positions, charges=np.ones(n), bounds=Quad(0, 0, 1),
+                                       k_e=1e-2, softening=1e-2, method="fmm")
+
+    sim = simulation(a.T)
+    for positions in (a.T, a.reshape(2, n), a.T):
+        sim.positions = positions
+        sim.compute_fields()
+        want = simulation(positions.clone(memory_format=torch.contiguous_format))
+        want.compute_fields()
+        assert relative(sim._electric.cpu().numpy(), want._electric.cpu().numpy()) < 1e-13
+    # a saved state of other strides (of an object kept from elsewhere) is compared as arrays
+    pos, *rest = sim._field_state
+    sim._field_state = (a.T, *rest)
+    sim.positions = a.reshape(2, n)
+    assert sim._electric.is_contiguous() and sim._scan() is None and not sim._fields_current()
+
+
 def test_velocities_that_autograd_follows_step_on_array_operations():
     sim = _simulation(50, 1.0, "free")
     sim.velocities.requires_grad_(True)

@@ -245,8 +245,10 @@ class ElectrostaticSimulation:
         last = [0, 0, 0]
         state = self._field_state
         if state is not None and state[0].shape == self.positions.shape:
-            if [t.dtype for t in state[:3]] != [torch.float64, torch.float64, torch.bool]:
-                return None  # fields of other arrays: compared as arrays
+            for saved, now in zip(state, (self.positions, self.charges, self.fixed)):
+                if (saved.dtype != now.dtype or saved.shape != now.shape
+                        or saved.device != now.device or not saved.is_contiguous()):
+                    return None  # fields of other arrays: compared as arrays
             last = [t.data_ptr() for t in state[:3]]
         axis = np.array([w[1] for w in self._walls], dtype=np.int32)
         sign = np.array([w[2] for w in self._walls], dtype=np.float64)
@@ -369,7 +371,9 @@ class ElectrostaticSimulation:
                 phi = phi + self._line_offset()
             self._potential = self.k_e * phi
         self._electric = self.k_e * self.charges[None, :] * field
-        self._field_state = (self.positions.clone(), self.charges.clone(), self.fixed.clone(),
+        # contiguous whatever the state's strides: _scan hands the copies to a kernel
+        self._field_state = (*(t.clone(memory_format=torch.contiguous_format)
+                               for t in (self.positions, self.charges, self.fixed)),
                              self._parameters())
         return self._tree
 
