@@ -103,6 +103,29 @@ def test_fields_of_a_transposed_state_are_not_taken_for_another_of_the_same_memo
     assert sim._electric.is_contiguous() and sim._scan() is None and not sim._fields_current()
 
 
+@pytest.mark.parametrize("kernel", ["coulomb", "log"])
+def test_direct_sums_of_a_strided_state(kernel):
+    """Direct fields and the exact pair energy of positions that are a transposed array and
+    charges that are every second one of an array."""
+    from tree_d_3d_b200 import Quad
+    from tree_d_3d_b200.simulation import ElectrostaticSimulation
+
+    n = 500
+    rng = np.random.default_rng(8)
+    a = torch.tensor(rng.uniform(-0.9, 0.9, (n, 2)), device="cuda")
+    q = torch.tensor(rng.normal(size=2 * n), device="cuda")[::2]
+    sims = [ElectrostaticSimulation(positions=a.T, charges=q, bounds=Quad(0, 0, 1), k_e=1e-2,
+                                    softening=1e-2, kernel=kernel) for _ in range(2)]
+    sims[0].positions, sims[0].charges = a.T, q
+    for include_fixed in (True, False):
+        for sim in sims:
+            sim._field_state = None
+            sim.compute_fields(include_fixed=include_fixed)
+        assert relative(sims[0]._electric.cpu().numpy(), sims[1]._electric.cpu().numpy()) < 1e-13
+    energy = [sim.get_potential_energy(exact=True) for sim in sims]
+    assert abs(energy[0] - energy[1]) <= 1e-12 * abs(energy[1])
+
+
 def test_velocities_that_autograd_follows_step_on_array_operations():
     sim = _simulation(50, 1.0, "free")
     sim.velocities.requires_grad_(True)

@@ -444,7 +444,8 @@ class ElectrostaticSimulation:
         status = status_word(dev)
         energy = torch.zeros(1, dtype=torch.float64, device=dev)
         ws = _lib.workspace(_lib.query("td3_pair_energy_workspace_size", n), dev)
-        _lib.call("td3_pair_energy", self.positions.data_ptr(), self.charges.data_ptr(), n,
+        pos, charge = _device(self.positions), _device(self.charges)
+        _lib.call("td3_pair_energy", pos.data_ptr(), charge.data_ptr(), n,
                   float(self.softening), energy.data_ptr(), status.data_ptr(), ws.data_ptr(),
                   ws.numel(), _lib.stream(dev))
         _check(status)
