@@ -193,3 +193,30 @@ def test_short_traversal_workspaces_are_refused():
             rc = lib.td3_fmm_traverse(0, 0, 0, 0, 0, nodes, 0.5, 0, 0, 0, 0, frontier,
                                       sizes.ctypes.data, 0, int(short), 0)
             assert rc == _lib.EWORKSPACE, (frontier, nodes, short)
+
+
+def test_simulation_kernels_take_arrays_of_one_gpu_only(monkeypatch):
+    """State on another GPU, or on the host, steps on array operations (where torch raises)."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from tree_d_3d_b200 import simulation
+    from tree_d_3d_b200.simulation import ElectrostaticSimulation, _one_gpu
+
+    on = [SimpleNamespace(device=torch.device(*d)) for d in (("cuda", 0), ("cuda", 1), ("cpu",))]
+    assert _one_gpu([on[0], on[0]]) and _one_gpu([on[1], on[1]])
+    assert not _one_gpu([on[0], on[1]])
+    assert not _one_gpu([on[0], on[2]])
+    assert not _one_gpu([on[2], on[2]])
+    # every array of the state is asked
+    sim = ElectrostaticSimulation.__new__(ElectrostaticSimulation)
+    for name in ("positions", "velocities", "_electric"):
+        setattr(sim, name, torch.zeros((2, 3), dtype=torch.float64))
+    sim.charges, sim.masses = torch.ones(3).double(), torch.ones(3).double()
+    sim.fixed = torch.zeros(3, dtype=torch.bool)
+    assert not sim._native()
+    asked = []
+    monkeypatch.setattr(simulation, "_one_gpu", lambda arrays: bool(asked.extend(arrays)))
+    assert not sim._native()
+    assert {id(a) for a in asked} == {id(a) for a in vars(sim).values()} and len(asked) == 6

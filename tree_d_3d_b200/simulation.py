@@ -101,6 +101,12 @@ def _drift(pos, vel, charges, masses, b_z, dt, mobile):
     return pos, vel
 
 
+def _one_gpu(arrays) -> bool:
+    """Whether the arrays are all on the same CUDA device."""
+    first = arrays[0].device
+    return first.type == "cuda" and all(a.device == first for a in arrays)
+
+
 class _Facts:
     """The state in numbers (td3_sim_scan): one host read for the questions that a step's
     host logic asks."""
@@ -227,15 +233,16 @@ class ElectrostaticSimulation:
         constructor makes them, and nothing that autograd follows); otherwise a step runs
         on array operations."""
         n, grad = self.num_particles, torch.is_grad_enabled()
-        for array, shape in ((self.positions, (2, n)), (self.velocities, (2, n)),
-                             (self._electric, (2, n)), (self.charges, (n,)),
-                             (self.masses, (n,)), (self.fixed, (n,))):
+        arrays = (self.positions, self.velocities, self._electric, self.charges, self.masses,
+                  self.fixed)
+        for array, shape in zip(arrays, 3 * ((2, n),) + 3 * ((n,),)):
             dtype = torch.bool if array is self.fixed else torch.float64
-            if (type(array) is not torch.Tensor or array.dtype != dtype or not array.is_cuda
+            if (type(array) is not torch.Tensor or array.dtype != dtype
                     or tuple(array.shape) != shape or not array.is_contiguous()
                     or (grad and array.requires_grad)):
                 return False
-        return True
+        # on two GPUs, or off the current one, torch takes or refuses them
+        return _one_gpu(arrays) and arrays[0].device.index == torch.cuda.current_device()
 
     def _scan(self) -> _Facts | None:
         """The state's facts (None where its arrays are not the kernels' kind)."""
