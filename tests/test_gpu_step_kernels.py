@@ -136,6 +136,54 @@ def test_velocities_that_autograd_follows_step_on_array_operations():
     assert v.grad is not None
 
 
+def test_forward_mode_tangents_of_a_step():
+    """Tangents of the velocities go through the array operations: with no charge and no
+    field a step moves by dt v."""
+    from torch.autograd import forward_ad
+
+    sim = _simulation(40, 0.0, "free")
+    sim.k_e = 0.0
+    tangent = torch.randn_like(sim.velocities)
+    with forward_ad.dual_level():
+        sim.velocities = forward_ad.make_dual(sim.velocities, tangent)
+        assert not sim._native()
+        sim.step()
+        moved = forward_ad.unpack_dual(sim.positions).tangent
+        assert torch.allclose(moved, sim.dt * tangent, rtol=1e-14, atol=0)
+    assert sim.velocities.is_cuda
+
+
+def test_step_under_torch_func_jvp():
+    sim = _simulation(40, 0.0, "free")
+    sim.k_e = 0.0
+    start, tangent = sim.velocities.clone(), torch.randn_like(sim.velocities)
+
+    def positions(velocities):
+        sim.velocities = velocities
+        sim.step()
+        return sim.positions
+
+    _, moved = torch.func.jvp(positions, (start,), (tangent,))
+    assert torch.allclose(moved, sim.dt * tangent, rtol=1e-14, atol=0)
+
+
+@pytest.mark.parametrize("shape", [(), (60,)])
+def test_magnetic_field_as_a_tensor(shape):
+    """B_z as a scalar or per-particle tensor: the array step, with gradients to it."""
+    sims = [_simulation(60, 1.25, "free") for _ in range(2)]
+    b_z = torch.full(shape, 1.25, dtype=torch.float64, device="cuda", requires_grad=True)
+    sims[1].B_z = b_z
+    assert sims[0]._native() and not sims[1]._native()
+    for sim in sims:
+        sim.step()
+    assert relative(sims[1].positions.detach().cpu().numpy(),
+                    sims[0].positions.cpu().numpy()) < 1e-13
+    assert relative(sims[1].velocities.detach().cpu().numpy(),
+                    sims[0].velocities.cpu().numpy()) < 1e-11
+    (grad,) = torch.autograd.grad(sims[1].positions.sum(), b_z)
+    assert grad.shape == b_z.shape and bool(grad.abs().sum() > 0)
+
+
 def test_pair_sum_logarithm_and_reciprocal():
     """direct_field of the log kernel at single distances: phi = -ln r^2 and E = 2 / r to a few
     units in the last place at every magnitude (the table's intervals, both sides of r = 1,

@@ -23,6 +23,7 @@ from collections.abc import Mapping
 
 import numpy as np
 import torch
+from torch.autograd import forward_ad
 
 from tree_d_3d_b200 import _lib
 from tree_d_3d_b200._utils import _check, _device, _finite, _points, device, status_word
@@ -99,6 +100,18 @@ def _drift(pos, vel, charges, masses, b_z, dt, mobile):
     pos = pos + step * mobile
     vel = torch.where(mobile.bool(), rotated, vel)
     return pos, vel
+
+
+def _differentiated(array: torch.Tensor) -> bool:
+    """Whether a transform other than reverse mode follows ``array``: a forward-mode tangent,
+    or a wrapper of torch.func (vmap, jvp, grad), which has no memory of its own."""
+    if forward_ad.unpack_dual(array).tangent is not None:
+        return True
+    try:
+        array.data_ptr()
+    except RuntimeError:
+        return True
+    return False
 
 
 def _one_gpu(arrays) -> bool:
@@ -230,8 +243,10 @@ class ElectrostaticSimulation:
 
     def _native(self) -> bool:
         """Whether the state's arrays are as the step's own kernels take them (as the
-        constructor makes them, and nothing that autograd follows); otherwise a step runs
-        on array operations."""
+        constructor makes them, and nothing that is differentiated) and B_z is a number;
+        otherwise a step runs on array operations."""
+        if not isinstance(self.B_z, (int, float)):
+            return False
         n, grad = self.num_particles, torch.is_grad_enabled()
         arrays = (self.positions, self.velocities, self._electric, self.charges, self.masses,
                   self.fixed)
@@ -239,7 +254,7 @@ class ElectrostaticSimulation:
             dtype = torch.bool if array is self.fixed else torch.float64
             if (type(array) is not torch.Tensor or array.dtype != dtype
                     or tuple(array.shape) != shape or not array.is_contiguous()
-                    or (grad and array.requires_grad)):
+                    or (grad and array.requires_grad) or _differentiated(array)):
                 return False
         # on two GPUs, or off the current one, torch takes or refuses them
         return _one_gpu(arrays) and arrays[0].device.index == torch.cuda.current_device()
