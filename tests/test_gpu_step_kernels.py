@@ -184,6 +184,34 @@ def test_magnetic_field_as_a_tensor(shape):
     assert grad.shape == b_z.shape and bool(grad.abs().sum() > 0)
 
 
+@pytest.mark.parametrize("how", ["subclass", "instance"])
+def test_step_calls_an_overridden_compute_fields(how):
+    """A program's own compute_fields (here: a uniform force added to the charges') gives both
+    half kicks of a step."""
+    from tree_d_3d_b200.simulation import ElectrostaticSimulation
+
+    class Tilted(ElectrostaticSimulation):
+        def compute_fields(self, include_fixed=True, potential=True):
+            self._field_state = None
+            tree = super().compute_fields(include_fixed, potential)
+            self._electric = self._electric + 3.0
+            return tree
+
+    sim = _simulation(30, 0.0, "free")
+    sim.k_e = 0.0
+    if how == "subclass":
+        sim.__class__ = Tilted
+    else:
+        def fields(include_fixed=True, potential=True):
+            sim._electric = torch.full_like(sim.positions, 3.0)
+
+        sim.compute_fields = fields
+    before = sim.velocities
+    sim.step()
+    assert torch.allclose(sim.velocities, before + sim.dt * 3.0 / sim.masses, rtol=1e-13, atol=1e-14)
+    assert torch.equal(sim.forces, torch.full_like(sim.forces, 3.0))
+
+
 def test_pair_sum_logarithm_and_reciprocal():
     """direct_field of the log kernel at single distances: phi = -ln r^2 and E = 2 / r to a few
     units in the last place at every magnitude (the table's intervals, both sides of r = 1,

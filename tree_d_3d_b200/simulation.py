@@ -243,9 +243,11 @@ class ElectrostaticSimulation:
 
     def _native(self) -> bool:
         """Whether the state's arrays are as the step's own kernels take them (as the
-        constructor makes them, and nothing that is differentiated) and B_z is a number;
+        constructor makes them, and nothing that is differentiated), B_z is a number and
+        compute_fields, which that step does not call a second time, is this class's;
         otherwise a step runs on array operations."""
-        if not isinstance(self.B_z, (int, float)):
+        if (not isinstance(self.B_z, (int, float)) or getattr(self.compute_fields, "__func__", None)
+                is not ElectrostaticSimulation.compute_fields):
             return False
         n, grad = self.num_particles, torch.is_grad_enabled()
         arrays = (self.positions, self.velocities, self._electric, self.charges, self.masses,
