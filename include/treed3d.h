@@ -242,7 +242,9 @@ int td3_evaluate_quadtree(int kernel, const double* targets, int64_t m, const in
  * the reference's serial order (generation by generation, frontier order); sizes
  * (HOST, 4) = n_m2l, n_p2p, next frontier, -1 on overflow, when TD3_ENEEDMORE is
  * returned (retry with larger buffers).  frontier_capacity bounds one generation.
- * Synchronises `stream` once per 8 generations.  Replaces fmm_traverse
+ * Synchronises `stream` after 16 generations, then once per 8.  A generation's blocks wait
+ * for one another's counts; a wait that runs out ends the call with TD3_ECUDA.  Replaces
+ * fmm_traverse
  * (src/tree_d_3d/kernels/fmm_traverse/fmm_traverse_pyccel.py:15-106,
  * fmm_traverse_cuda.cu:14-97) driven by FlatQuadtree._traverse
  * (src/tree_d_3d/flat_tree.py:1318-1358); identical lists.  n_nodes: the node count
@@ -254,6 +256,15 @@ int td3_fmm_traverse(const double* node_center, const double* node_half,
                      int64_t m2l_capacity, int64_t* p2p, int64_t p2p_capacity,
                      int64_t frontier_capacity, int64_t* sizes, void* workspace,
                      size_t workspace_bytes, void* stream);
+
+/* td3_fmm_traverse with waits of at most `polls` polls (0 to 4194304, its own number): with 0
+ * they run out at once, which is how a program tests what it does then. */
+int td3_fmm_traverse_polls(const double* node_center, const double* node_half,
+                           const int64_t* node_start, const int64_t* node_end,
+                           const int64_t* node_child, int64_t n_nodes, double theta, int64_t* m2l,
+                           int64_t m2l_capacity, int64_t* p2p, int64_t p2p_capacity,
+                           int64_t frontier_capacity, int64_t* sizes, int64_t polls,
+                           void* workspace, size_t workspace_bytes, void* stream);
 
 /* The one-way traversal of a target tree (t_*) against a source tree (s_*) from
  * (root, root), with the predicates of td3_fmm_traverse; pairs are (target cell,

@@ -87,7 +87,9 @@ __device__ __forceinline__ int classify_dual(i64 a, i64 b, const NodeRec* __rest
 // tiles before it: their counts up to the nearest one whose own first slots are known
 // (Merrill and Garland's decoupled look-back).  Tiles are taken in order by resident blocks,
 // so a tile's predecessors are always under way; the wait for them is bounded all the same
-// (LOOK_LIMIT polls, then the state's `failed`, which the host turns into an error).
+// (LOOK_LIMIT polls, then the state's `failed`, which the host turns into an error).  One
+// thread reads for its block what the other blocks may write meanwhile (`failed`, a ticket),
+// so that the block goes on or leaves as a whole.
 //
 // Measured (all generations of theta 0.5, host reads included) against two launches per
 // generation, one that classifies and scans and one that reads the frontier again and emits:
@@ -149,15 +151,17 @@ __device__ __forceinline__ void store_release(unsigned* p, unsigned v) {
 
 // The counts of all tiles before `tile` (one warp; every lane returns them): 32 tiles at a
 // time, the lanes nearest first, up to the nearest tile whose `all` is there.
-__device__ TileCounts look_back(TileState* state, i64 tile, unsigned own_ready, bool* failed) {
+__device__ TileCounts look_back(TileState* state, i64 tile, unsigned own_ready, unsigned limit,
+                                bool* failed) {
     const int lane = threadIdx.x & 31;
     TileCounts sum{0, 0};
     for (i64 at = tile - 1; at >= 0; at -= 32) {
         const i64 t = at - lane;
         unsigned ready = own_ready + 1;  // before the first tile: nothing, known
         if (t >= 0) {
-            unsigned polls = 0;
-            while ((ready = load_acquire(&state[t].ready)) < own_ready && ++polls < LOOK_LIMIT)
+            ready = 0;
+            for (unsigned polls = 0;
+                 polls < limit && (ready = load_acquire(&state[t].ready)) < own_ready; ++polls)
                 __nanosleep(20);
         }
         if (__any_sync(0xffffffffu, ready < own_ready)) {
@@ -188,14 +192,14 @@ __device__ TileCounts look_back(TileState* state, i64 tile, unsigned own_ready, 
 // pair first + 32 r + l); ballots rank a round's outputs, in frontier order.
 template <bool DUAL>
 __global__ void __launch_bounds__(TRAV_THREADS, GEN_BLOCKS)
-k_generation(const FPair* __restrict__ frontier, TravState* st, int gen,
+k_generation(const FPair* __restrict__ frontier, TravState* st, int gen, unsigned look_limit,
              const NodeRec* __restrict__ t_rec, const NodeRec* __restrict__ s_rec, double theta,
              TileState* tile_state, Pair* __restrict__ m2l, i64 m2l_capacity,
              Pair* __restrict__ p2p, i64 p2p_capacity, FPair* __restrict__ next,
              i64 frontier_capacity) {
     constexpr int WARPS = TRAV_THREADS / 32;
     __shared__ unsigned warp_m2l[WARPS], warp_p2p[WARPS], warp_next[WARPS];
-    __shared__ i64 base_m2l_s, base_p2p_s, base_next_s;
+    __shared__ i64 base_m2l_s, base_p2p_s, base_next_s, nf_s, listed_m2l_s, listed_p2p_s;
     __shared__ unsigned taken;
     td3_chain_wait();
     td3_chain_release();
@@ -203,7 +207,14 @@ k_generation(const FPair* __restrict__ frontier, TravState* st, int gen,
     const unsigned before = (1u << lane) - 1u;
     // read before this block takes a tile: the last tile's block moves them on (a generation
     // after a failed one, whose frontier has holes, is empty)
-    const i64 nf = st->failed ? 0 : st->nf[parity], listed_m2l = st->n_m2l, listed_p2p = st->n_p2p;
+    if (threadIdx.x == 0) {
+        const i64 size = st->nf[parity], m = st->n_m2l, p = st->n_p2p, stop = st->failed;
+        nf_s = stop ? 0 : size;
+        listed_m2l_s = m;
+        listed_p2p_s = p;
+    }
+    __syncthreads();
+    const i64 nf = nf_s, listed_m2l = listed_m2l_s, listed_p2p = listed_p2p_s;
     const i64 tiles = (nf + GEN_TILE - 1) / GEN_TILE;
     const unsigned own_ready = 2u * (unsigned)gen + 1u;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -257,7 +268,7 @@ k_generation(const FPair* __restrict__ frontier, TravState* st, int gen,
                 store_release(&mine->ready, own_ready);
             }
             bool failed = false;
-            const TileCounts pre = look_back(tile_state, tile, own_ready, &failed);
+            const TileCounts pre = look_back(tile_state, tile, own_ready, look_limit, &failed);
             if (lane == 0) {
                 const TileCounts all{pre.lists + own.lists, pre.next + own.next};
                 if (failed) {
@@ -385,7 +396,8 @@ int launch_records(i64 count, const double* center, const double* half, const i6
 template <bool DUAL>
 int run_generations(const NodeRec* t, const NodeRec* s, double theta, Pair* m2l,
                     i64 m2l_capacity, Pair* p2p, i64 p2p_capacity, i64 frontier_capacity,
-                    int64_t* sizes, const TraverseBuffers& b, cudaStream_t stream) {
+                    int64_t* sizes, const TraverseBuffers& b, unsigned look_limit,
+                    cudaStream_t stream) {
     i64 tiles = gen_tiles(frontier_capacity);
     unsigned grid = (unsigned)(tiles < 148 * 4 ? tiles : 148 * 4);
     TD3_TRY(td3_launch_chained(k_gen_init, td3_blocks(tiles, 256), 256, 0, stream, b.state,
@@ -396,8 +408,8 @@ int run_generations(const NodeRec* t, const NodeRec* s, double theta, Pair* m2l,
         for (const int stop = gen + (gen ? GEN_BATCH : GEN_FIRST); gen < stop; ++gen) {
             const int parity = gen & 1;
             TD3_TRY(td3_launch_chained(k_generation<DUAL>, grid, TRAV_THREADS, 0, stream,
-                                       (const FPair*)b.frontier[parity], b.state, gen, t, s,
-                                       theta, b.tile, m2l, m2l_capacity, p2p, p2p_capacity,
+                                       (const FPair*)b.frontier[parity], b.state, gen, look_limit,
+                                       t, s, theta, b.tile, m2l, m2l_capacity, p2p, p2p_capacity,
                                        b.frontier[parity ^ 1], frontier_capacity));
         }
         TD3_CHECK_LAUNCH();
@@ -481,14 +493,15 @@ extern "C" size_t td3_fmm_traverse_workspace_size(int64_t frontier_capacity, int
     return traverse_workspace(frontier_capacity, n_nodes);
 }
 
-extern "C" int td3_fmm_traverse(const double* node_center, const double* node_half,
-                                const int64_t* node_start, const int64_t* node_end,
-                                const int64_t* node_child, int64_t n_nodes, double theta,
-                                int64_t* m2l, int64_t m2l_capacity, int64_t* p2p,
-                                int64_t p2p_capacity, int64_t frontier_capacity, int64_t* sizes,
-                                void* workspace, size_t workspace_bytes, void* stream) {
+extern "C" int td3_fmm_traverse_polls(const double* node_center, const double* node_half,
+                                      const int64_t* node_start, const int64_t* node_end,
+                                      const int64_t* node_child, int64_t n_nodes, double theta,
+                                      int64_t* m2l, int64_t m2l_capacity, int64_t* p2p,
+                                      int64_t p2p_capacity, int64_t frontier_capacity,
+                                      int64_t* sizes, int64_t polls, void* workspace,
+                                      size_t workspace_bytes, void* stream) {
     if (frontier_capacity < 1 || m2l_capacity < 0 || p2p_capacity < 0) return TD3_EINVAL;
-    if (n_nodes < 1 || n_nodes > 0x7fffffffLL) return TD3_EINVAL;
+    if (n_nodes < 1 || n_nodes > 0x7fffffffLL || polls < 0 || polls > LOOK_LIMIT) return TD3_EINVAL;
     Workspace w(workspace, workspace_bytes);
     TraverseBuffers b;
     if (!take_traverse(w, frontier_capacity, n_nodes, 0, b)) return TD3_EWORKSPACE;
@@ -497,7 +510,18 @@ extern "C" int td3_fmm_traverse(const double* node_center, const double* node_ha
                               b.rec[0], s));
     return run_generations<false>(b.rec[0], b.rec[0], theta, reinterpret_cast<Pair*>(m2l),
                                   m2l_capacity, reinterpret_cast<Pair*>(p2p), p2p_capacity,
-                                  frontier_capacity, sizes, b, s);
+                                  frontier_capacity, sizes, b, (unsigned)polls, s);
+}
+
+extern "C" int td3_fmm_traverse(const double* node_center, const double* node_half,
+                                const int64_t* node_start, const int64_t* node_end,
+                                const int64_t* node_child, int64_t n_nodes, double theta,
+                                int64_t* m2l, int64_t m2l_capacity, int64_t* p2p,
+                                int64_t p2p_capacity, int64_t frontier_capacity, int64_t* sizes,
+                                void* workspace, size_t workspace_bytes, void* stream) {
+    return td3_fmm_traverse_polls(node_center, node_half, node_start, node_end, node_child, n_nodes,
+                                  theta, m2l, m2l_capacity, p2p, p2p_capacity, frontier_capacity,
+                                  sizes, LOOK_LIMIT, workspace, workspace_bytes, stream);
 }
 
 extern "C" int td3_dual_traverse(const double* t_center, const double* t_half,
@@ -519,7 +543,7 @@ extern "C" int td3_dual_traverse(const double* t_center, const double* t_half,
     TD3_TRY_RC(launch_records(s_nodes, s_center, s_half, s_start, s_end, s_child, b.rec[1], s));
     return run_generations<true>(b.rec[0], b.rec[1], theta, reinterpret_cast<Pair*>(m2l),
                                  m2l_capacity, reinterpret_cast<Pair*>(p2p), p2p_capacity,
-                                 frontier_capacity, sizes, b, s);
+                                 frontier_capacity, sizes, b, LOOK_LIMIT, s);
 }
 
 extern "C" size_t td3_pair_csr_workspace_size(int64_t count, int mutual, int64_t n_nodes) {
