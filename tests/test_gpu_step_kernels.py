@@ -233,3 +233,57 @@ def test_pair_sum_logarithm_and_reciprocal():
         finite = np.isfinite(ref)  # 2 / r^2 of a denormal r^2 is infinite
         assert np.array_equal(got[~finite], ref[~finite])
         assert np.all(np.abs(got[finite] - ref[finite]) <= 4 * np.spacing(np.abs(ref[finite])))
+
+
+@pytest.mark.parametrize("sources", [1, 2, 3])
+def test_pair_sum_reciprocal_root(sources):
+    """direct_field of the Coulomb kernel at single distances: phi = 1 / r and E = 1 / r^2 over
+    all magnitudes, past the largest and smallest normal r^2, beside sources without charge (the
+    pairs are summed two at a time).  Units in the last place: 1 for the root of the rounded
+    r^2 (half of r^2's half, and the function's 1 at most), E three of those and three products."""
+    from tree_d_3d_b200 import direct_field
+
+    rng = np.random.default_rng(1)
+    near = 1 + np.concatenate([s * 2.0 ** -np.arange(1.0, 50.0) for s in (1, -1)])
+    r = np.concatenate([np.exp(rng.uniform(-300, 300, 20000)), rng.uniform(0.5, 2, 20000), near,
+                        2.0 ** np.arange(-530, 505.0), [1.0, 1e-155, 1e-160, 1e153, 1e154, 1e160]])
+    source = np.zeros((2, sources))
+    charge = np.zeros(sources)
+    charge[sources // 2] = 1.0
+    phi, field = direct_field(torch.tensor(np.stack((r, 0 * r)), device="cuda"),
+                              torch.tensor(source, device="cuda"),
+                              torch.tensor(charge, device="cuda"))
+    with np.errstate(over="ignore"):
+        r2 = r * r
+        want = 1 / np.sqrt(r2.astype(np.longdouble))
+        cube = (want.astype(np.float64) ** 3).astype(np.longdouble) * r
+    for got, ref, units in ((phi, want, 2), (field[0], cube, 8)):
+        got, ref = got.cpu().numpy(), ref.astype(np.float64)
+        normal = np.isfinite(ref) & (ref >= 2.0 ** -1000)
+        if units == 8:  # 1 / r^3 is normal, too
+            normal &= (r < 1e102) & (r > 1e-102)
+        assert np.all(np.abs(got[normal] - ref[normal]) <= units * np.spacing(ref[normal]))
+        assert not np.isnan(got[r2 > 0]).any()
+    big = np.isinf(r2)
+    assert big.any() and not phi.cpu().numpy()[big].any()
+
+
+@pytest.mark.parametrize("call", ["direct", "walk", "fmm"])
+def test_log_pairs_beyond_the_reciprocals_range(call):
+    """E = 2 q d / r^2 of line charges whose 1 / r^2 alone would overflow, or be denormal."""
+    from tree_d_3d_b200 import FlatQuadtree, Quad, direct_field
+
+    for r, q in ((1e-157, 1e-200), (3e-156, 1e-180), (1e-100, 1e-250), (1e153, 1e200), (7e153, 1e250)):
+        pos = np.array([[0.0, r], [0.0, 0.0]])
+        charge = np.full(2, q)
+        if call == "direct":
+            phi, field = direct_field(pos, pos, charge, exclude=np.arange(2), kernel="log")
+        else:
+            tree = FlatQuadtree(pos, charge, Quad(0, 0, 4 * r), kernel="log", order=2)
+            phi, field = (tree.fmm() if call == "fmm" else
+                          tree.evaluate(pos, exclude=np.arange(2)))
+        r2 = r * r  # denormal for the first two
+        want = 2 * q / r2 * r
+        assert np.isfinite(want) and abs(want) > 0
+        assert np.all(np.abs(field[0] - [-want, want]) <= 8 * np.spacing(want)), (r, q)
+        assert np.all(np.abs(phi + q * np.log(r2)) <= 8 * np.spacing(abs(q * np.log(r2))))

@@ -7,9 +7,9 @@
 // workspace, reduced afterwards in a fixed order (deterministic results).
 //
 // The FP64 pipe bounds it: two sources at a time, so that one pair's chain of operations
-// fills the other's waits, and math64.cuh's functions in place of the library's.  4096
-// targets of 200,000 line charges, whole call: 4.03 ms with the library's functions and one
-// source at a time, 2.61 with math64.cuh's, 2.43 ms with two sources.
+// fills the other's waits, and math64.cuh's logarithm and reciprocal in place of the library's.
+// 4096 targets of 200,000 line charges, whole call: 4.03 ms with the library's functions and one
+// source at a time, 2.61 ms so.
 #include <mutex>
 
 #include "common.cuh"
@@ -26,7 +26,7 @@ k_direct(const double* __restrict__ targets, i64 m, const i64* __restrict__ excl
          const double* __restrict__ pos, const double* __restrict__ charge, i64 n, i64 chunk,
          double eps2, double* __restrict__ phi, double* __restrict__ field,
          double* __restrict__ partial, i64* status) {
-    constexpr bool LOG = KERNEL == TD3_KERNEL_LOG && POT;
+    constexpr bool LOG = KERNEL == TD3_KERNEL_LOG;
     __shared__ double sx[DIRECT_THREADS], sy[DIRECT_THREADS], sq[DIRECT_THREADS];
     __shared__ double2 table[LOG ? LOG64_SIZE : 1];
     if (LOG) fill_log64(table);  // read after the first tile's barrier
@@ -62,32 +62,32 @@ k_direct(const double* __restrict__ targets, i64 m, const i64* __restrict__ excl
                 cb[u] = none ? 0.0 : c;
                 r2[u] = none ? 1.0 : dx[u] * dx[u] + dy[u] * dy[u] + eps2;
                 bad |= (r2[u] == 0.0);
-                if (KERNEL == TD3_KERNEL_COULOMB) {
-                    inv[u] = rsqrt64(r2[u]);
-                } else {
-                    inv[u] = reciprocal64(r2[u]);
-                    if (POT) ln[u] = log64(r2[u], table);
-                }
+                if (LOG)
+                    log_reciprocal64<POT>(r2[u], table, ln[u], inv[u]);
+                else
+                    inv[u] = rsqrt(r2[u]);
             }
-            if (!in_range64(r2[0]) || !in_range64(r2[1])) {
+            double f[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) f[u] = 2.0 * cb[u] * inv[u];
+            if (LOG && (!in_range64(r2[0]) || !in_range64(r2[1]))) {
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
-                    inv[u] = KERNEL == TD3_KERNEL_COULOMB ? rsqrt(r2[u]) : 1.0 / r2[u];
-                    if (LOG) ln[u] = log(r2[u]);
+                    f[u] = 2.0 * cb[u] / r2[u];
+                    if (POT) ln[u] = log(r2[u]);
                 }
             }
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
-                if (KERNEL == TD3_KERNEL_COULOMB) {
+                if (LOG) {
+                    if (POT) p -= cb[u] * ln[u];
+                    ex += f[u] * dx[u];
+                    ey += f[u] * dy[u];
+                } else {
                     const double inv_r3 = inv[u] * inv[u] * inv[u];
                     p += cb[u] * inv[u];
                     ex += cb[u] * inv_r3 * dx[u];
                     ey += cb[u] * inv_r3 * dy[u];
-                } else {
-                    if (POT) p -= cb[u] * ln[u];
-                    const double f = 2.0 * cb[u] * inv[u];
-                    ex += f * dx[u];
-                    ey += f * dy[u];
                 }
             }
         }
@@ -185,7 +185,7 @@ k_pair_energy(const double* __restrict__ pos, const double* __restrict__ charge,
             double dx = xi - sx[t], dy = yi - sy[t];
             double r2 = dx * dx + dy * dy + eps2;
             bad |= (r2 == 0.0 && qi != 0.0);
-            row += cj * rsqrt_any(r2);
+            row += cj * rsqrt(r2);
         }
         __syncthreads();
     }

@@ -12,7 +12,6 @@
 // with one segment writes its final values; the segments of a longer row write
 // partial sums that a finish pass adds in segment order (deterministic results).
 #include "common.cuh"
-#include "math64.cuh"
 
 namespace {
 
@@ -388,7 +387,7 @@ k_near(Targets T, Sources S, i64 n_seg, const int* __restrict__ seg_leaf,
                 }
             } else {
                 // no branches but the rare ones: the chains of two pairs overlap (a step
-                // of 1M charges, 3.30 -> 3.22 ms)
+                // of 1M charges, 3.30 -> 3.25 ms)
 #pragma unroll 2
                 for (int p = slice; p < wn; p += slices) {
                     const double q0 = win.q[p];
@@ -405,11 +404,11 @@ k_near(Targets T, Sources S, i64 n_seg, const int* __restrict__ seg_leaf,
                     const double qj = none ? 0.0 : q0;
                     if (KERNEL == TD3_KERNEL_LOG) {
                         if (POT) pot -= qj * log(r2);
-                        const double f = 2.0 * qj * reciprocal_any(r2);
+                        const double f = 2.0 * qj / r2;
                         ex += f * dx;
                         ey += f * dy;
                     } else {
-                        const double inv_r = rsqrt_any(r2);
+                        const double inv_r = rsqrt(r2);
                         const double qr3 = qj * (inv_r * inv_r * inv_r);
                         pot += qj * inv_r;
                         ex += qr3 * dx;
@@ -575,7 +574,7 @@ __device__ __forceinline__ void adjoint_pair(double dx, double dy, double eps2, 
     double de = exj * dx + eyj * dy;
     if (KERNEL == TD3_KERNEL_LOG) {
         // G = -ln s, grad G = -2 d / s, Hess G = -2 I / s + 4 d d^T / s^2
-        double inv = reciprocal_any(s);
+        double inv = 1.0 / s;
         double lg = log(s);
         acc[0] += -wj * lg - 2.0 * de * inv;
         double t = 4.0 * de * inv * inv;
@@ -587,7 +586,7 @@ __device__ __forceinline__ void adjoint_pair(double dx, double dy, double eps2, 
         acc[5] += -2.0 * qj * inv + q4 * dy * dy;
     } else {
         // G = s^(-1/2), grad G = -d s^(-3/2), Hess G = -I s^(-3/2) + 3 d d^T s^(-5/2)
-        double r = rsqrt_any(s);
+        double r = rsqrt(s);
         double r3 = r * r * r;
         double r5 = r3 * r * r;
         acc[0] += wj * r - de * r3;

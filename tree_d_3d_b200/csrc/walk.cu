@@ -13,7 +13,6 @@
 // descends while any lane needs the children.  Node data is packed per node for
 // broadcast loads.
 #include "common.cuh"
-#include "math64.cuh"
 
 namespace {
 
@@ -88,7 +87,7 @@ __device__ __forceinline__ bool inside_cell(double tx, double ty, double cx, dou
 // from d2 = |r|^2: decided by the squares where they differ by more than the roundings of
 // either form can (2^-48 of them; theta2 = theta^2), else by the test itself.  Without the
 // square root at every visit and with a leaf's particles two at a time, whole calls: 5000
-// targets 690 -> 633 us, 1M 4381 -> 4300 us (300k targets: 2.4 instructions a cycle, 47 % of
+// targets 690 -> 638 us, 1M 4381 -> 4300 us (300k targets: 2.4 instructions a cycle, 47 % of
 // the FP64 pipe in use).
 __device__ __forceinline__ bool far_enough(double h, double d2, double theta, double theta2) {
     const double s = 4.0 * h * h, t = theta2 * d2;
@@ -158,11 +157,7 @@ k_walk_coulomb(const double* __restrict__ targets, i64 m, const i64* __restrict_
                             if (none) c[u] = dx[u] = dy[u] = 0.0;
                             r2[u] = none ? 1.0 : dx[u] * dx[u] + dy[u] * dy[u] + eps2;
                             bad |= r2[u] == 0.0;
-                            ir[u] = rsqrt64(r2[u]);
-                        }
-                        if (!in_range64(r2[0]) || !in_range64(r2[1])) {
-                            ir[0] = rsqrt(r2[0]);
-                            ir[1] = rsqrt(r2[1]);
+                            ir[u] = rsqrt(r2[u]);
                         }
 #pragma unroll
                         for (int u = 0; u < 2; ++u) {
@@ -227,7 +222,7 @@ k_walk_coulomb(const double* __restrict__ targets, i64 m, const i64* __restrict_
                     double2 q89 = *reinterpret_cast<const double2*>(nd + 8);
                     double q = q45.x, px = q45.y, py = q67.x, sxx = q67.y, sxy = q89.x,
                            syy = q89.y;
-                    double inv_r = rsqrt_any(d2 + eps2);
+                    double inv_r = rsqrt(d2 + eps2);
                     double inv_r2 = inv_r * inv_r;
                     double inv_r3 = inv_r2 * inv_r;
                     double inv_r5 = inv_r3 * inv_r2;
@@ -349,7 +344,7 @@ k_walk_log(const double* __restrict__ targets, i64 m, const i64* __restrict__ ex
                         break;
                     }
                     if (POT) pot -= c * log(r2);
-                    double f = 2.0 * c * reciprocal_any(r2);
+                    double f = 2.0 * c / r2;
                     ex += f * dx;
                     ey += f * dy;
                 }
