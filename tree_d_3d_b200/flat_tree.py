@@ -52,7 +52,9 @@ def _direct(targets, exclude, pos, charge, softening, kernel, potential=True):
     """Device tensors in, (phi, field) device tensors out; raises on coincidence."""
     dev = targets.device
     # a simulation's arrays come as their user set them: strided, or of another type
-    targets, pos, charge = (t.to(torch.float64).contiguous() for t in (targets, pos, charge))
+    targets, pos, charge = (
+        t if t.dtype is torch.float64 and t.is_contiguous() else t.to(torch.float64).contiguous()
+        for t in (targets, pos, charge))
     m, n = targets.shape[1], pos.shape[1]
     phi = torch.zeros(m, dtype=torch.float64, device=dev)
     field = torch.zeros((2, m), dtype=torch.float64, device=dev)

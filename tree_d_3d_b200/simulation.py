@@ -102,13 +102,16 @@ def _drift(pos, vel, charges, masses, b_z, dt, mobile):
     return pos, vel
 
 
-def _differentiated(array: torch.Tensor) -> bool:
-    """Whether a transform other than reverse mode follows ``array``: a forward-mode tangent,
-    or a wrapper of torch.func (vmap, jvp, grad), which has no memory of its own."""
-    if forward_ad.unpack_dual(array).tangent is not None:
-        return True
+def _differentiated(arrays) -> bool:
+    """Whether a transform other than reverse mode follows one of the arrays: a forward-mode
+    tangent, or a wrapper of torch.func (vmap, jvp, grad), which has no memory of its own."""
+    # outside every dual level (-1) no tensor has a tangent
+    if getattr(forward_ad, "_current_level", 0) >= 0:
+        if any(forward_ad.unpack_dual(a).tangent is not None for a in arrays):
+            return True
     try:
-        array.data_ptr()
+        for a in arrays:
+            a.data_ptr()
     except RuntimeError:
         return True
     return False
@@ -249,21 +252,22 @@ class ElectrostaticSimulation:
         if (not isinstance(self.B_z, (int, float)) or getattr(self.compute_fields, "__func__", None)
                 is not ElectrostaticSimulation.compute_fields):
             return False
-        n, grad = self.num_particles, torch.is_grad_enabled()
+        n, grad, f64 = self.num_particles, torch.is_grad_enabled(), torch.float64
         arrays = (self.positions, self.velocities, self._electric, self.charges, self.masses,
                   self.fixed)
-        for array, shape in zip(arrays, 3 * ((2, n),) + 3 * ((n,),)):
-            dtype = torch.bool if array is self.fixed else torch.float64
-            if (type(array) is not torch.Tensor or array.dtype != dtype
-                    or tuple(array.shape) != shape or not array.is_contiguous()
-                    or (grad and array.requires_grad) or _differentiated(array)):
+        for array, shape, dtype in zip(arrays, 3 * ((2, n),) + 3 * ((n,),), 5 * (f64,) + (torch.bool,)):
+            if (type(array) is not torch.Tensor or array.dtype is not dtype
+                    or array.shape != shape or not array.is_contiguous()
+                    or (grad and array.requires_grad)):
                 return False
         # on two GPUs, or off the current one, torch takes or refuses them
-        return _one_gpu(arrays) and arrays[0].device.index == torch.cuda.current_device()
+        return (_one_gpu(arrays) and arrays[0].device.index == torch.cuda.current_device()
+                and not _differentiated(arrays))
 
-    def _scan(self) -> _Facts | None:
-        """The state's facts (None where its arrays are not the kernels' kind)."""
-        if not self._native():
+    def _scan(self, native: bool | None = None) -> _Facts | None:
+        """The state's facts (None where its arrays are not the kernels' kind; ``native``:
+        already asked)."""
+        if not (self._native() if native is None else native):
             return None
         n, dev = self.num_particles, self.positions.device
         last = [0, 0, 0]
@@ -434,9 +438,9 @@ class ElectrostaticSimulation:
                   self.fixed.data_ptr(), n, self.dt, self.B_z, pos.data_ptr(), vel.data_ptr(),
                   stream)
         self.positions, self.velocities = pos, vel
-        facts = self._scan()
+        facts = self._scan(True)
         if self._absorb(facts):
-            facts = self._scan()
+            facts = self._scan(True)
         tree = self._compute_fields(False, False, facts)
         vel, forces = torch.empty_like(self.velocities), torch.empty_like(self.positions)
         _lib.call("td3_sim_kick_force", self.velocities.data_ptr(), self._electric.data_ptr(),
