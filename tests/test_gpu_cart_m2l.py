@@ -55,10 +55,19 @@ def _oracle_locals(oracle, c, order, start=None, dst_center=None):
     return local
 
 
-def _run(c, order, mixed, packed):
+def _off_by_a_double(t):
+    """A copy of ``t`` that starts 8 bytes past a 16-byte boundary."""
+    copy = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)[1:].view_as(t)
+    assert copy.data_ptr() % 16 == 8
+    return copy.copy_(t)
+
+
+def _run(c, order, mixed, packed, shift=False):
     from tree_d_3d_b200 import _lib
 
     d = {k: torch.tensor(v, device="cuda") for k, v in c.items() if isinstance(v, np.ndarray)}
+    if shift:
+        d = {k: _off_by_a_double(v) for k, v in d.items()}
     n_dst, n_src = c["start"].size - 1, c["src_center"].shape[0]
     local = torch.zeros((n_dst, c["degree"].size), dtype=torch.float64, device="cuda")
     cells = (d["start"].data_ptr(), d["partners"].data_ptr(), n_dst, d["dst_center"].data_ptr(),
@@ -106,6 +115,14 @@ def test_cartesian_m2l_rows_match_the_oracle(oracle, order, eps):
         assert np.array_equal(packed, _run(c, order, mixed, True))  # the same bits every run
         assert error(_run(c, order, mixed, False), packed, mixed) < tol
         assert not packed[~filled].any()
+
+
+@pytest.mark.parametrize("order", [3, 12, 16])
+@pytest.mark.parametrize("mixed,packed", [(0, False), (0, True), (1, False), (1, True)])
+def test_arrays_on_any_double(order, mixed, packed):
+    """Rows, partners, centres, sizes and moments that start 8 bytes past a 16-byte boundary."""
+    c = _case(order, 1e-3, order)
+    assert np.array_equal(_run(c, order, mixed, packed, shift=True), _run(c, order, mixed, packed))
 
 
 def test_cartesian_records_reject_other_orders():

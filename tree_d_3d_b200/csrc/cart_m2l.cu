@@ -359,10 +359,9 @@ k_m2l_cart_rows(const i64* __restrict__ row_start, const i64* __restrict__ partn
     double tx = 0.0, ty = 0.0, hs = 0.0, hd = 1.0;
     auto fetch = [&](int src, i64 d) {
         if (src >= 0) {
-            const double2 c = reinterpret_cast<const double2*>(src_center)[src];
-            const double2 cd = reinterpret_cast<const double2*>(dst_center)[d];
-            tx = cd.x - c.x;
-            ty = cd.y - c.y;
+            // two 8-byte reads each: a caller's centres may start on any double
+            tx = dst_center[2 * d] - src_center[2 * (i64)src];
+            ty = dst_center[2 * d + 1] - src_center[2 * (i64)src + 1];
             if (MIXED) {
                 hs = src_half[src];
                 hd = dst_half[d];
