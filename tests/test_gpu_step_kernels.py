@@ -100,7 +100,7 @@ def test_fields_of_a_transposed_state_are_not_taken_for_another_of_the_same_memo
     pos, *rest = sim._field_state
     sim._field_state = (a.T, *rest)
     sim.positions = a.reshape(2, n)
-    assert sim._electric.is_contiguous() and sim._scan() is None and not sim._fields_current()
+    assert sim._native() and sim._scan() is None and not sim._fields_current()
 
 
 @pytest.mark.parametrize("kernel", ["coulomb", "log"])

@@ -215,7 +215,7 @@ def test_simulation_kernels_take_arrays_of_one_gpu_only(monkeypatch):
         setattr(sim, name, torch.zeros((2, 3), dtype=torch.float64))
     sim.charges, sim.masses = torch.ones(3).double(), torch.ones(3).double()
     sim.fixed = torch.zeros(3, dtype=torch.bool)
-    sim.B_z = 0.0
+    sim.B_z, sim.k_e = 0.0, 1.0
     assert not sim._native()
     asked = []
     monkeypatch.setattr(simulation, "_one_gpu", lambda arrays: bool(asked.extend(arrays)))

@@ -246,10 +246,11 @@ class ElectrostaticSimulation:
 
     def _native(self) -> bool:
         """Whether the state's arrays are as the step's own kernels take them (as the
-        constructor makes them, and nothing that is differentiated), B_z is a number and
-        compute_fields, which that step does not call a second time, is this class's;
-        otherwise a step runs on array operations."""
-        if (not isinstance(self.B_z, (int, float)) or getattr(self.compute_fields, "__func__", None)
+        constructor makes them, and nothing that is differentiated), B_z and k_e are numbers
+        and compute_fields, which that step does not call, is this class's; otherwise a step
+        runs on array operations.  Fields computed of such a state leave it such a state."""
+        if (not isinstance(self.B_z, (int, float)) or not isinstance(self.k_e, (int, float))
+                or getattr(self.compute_fields, "__func__", None)
                 is not ElectrostaticSimulation.compute_fields):
             return False
         n, grad, f64 = self.num_particles, torch.is_grad_enabled(), torch.float64
@@ -264,11 +265,8 @@ class ElectrostaticSimulation:
         return (_one_gpu(arrays) and arrays[0].device.index == torch.cuda.current_device()
                 and not _differentiated(arrays))
 
-    def _scan(self, native: bool | None = None) -> _Facts | None:
-        """The state's facts (None where its arrays are not the kernels' kind; ``native``:
-        already asked)."""
-        if not (self._native() if native is None else native):
-            return None
+    def _scan(self) -> _Facts | None:
+        """The facts of a state that is _native (None where the saved one is of another kind)."""
         n, dev = self.num_particles, self.positions.device
         last = [0, 0, 0]
         state = self._field_state
@@ -355,7 +353,8 @@ class ElectrostaticSimulation:
     def compute_fields(self, include_fixed: bool = True, potential: bool = True):
         """Electric force and potential on every particle, reused while the state is
         unchanged (simulation.py:704-798).  Returns the tree used (None: direct)."""
-        return self._compute_fields(include_fixed, potential, self._scan())
+        facts = self._scan() if self._native() else None
+        return self._compute_fields(include_fixed, potential, facts)
 
     def _compute_fields(self, include_fixed: bool, potential: bool, facts: _Facts | None):
         want_potential = potential or self.kernel != "log"
@@ -410,10 +409,10 @@ class ElectrostaticSimulation:
         """Electric half kick, exact cyclotron drift, absorption, electric half kick
         (simulation.py:800-835).  Returns the tree of the end-of-step forces."""
         self.dt = _finite("dt", self.dt if dt is None else dt, positive=True)
-        self.compute_fields(include_fixed=False, potential=False)
         if self._native():
             tree = self._native_step()
         else:
+            self.compute_fields(include_fixed=False, potential=False)
             mobile = (~self.fixed).to(torch.float64)
             self.velocities = self.velocities + 0.5 * self.dt * self._electric / self.masses * mobile
             self.positions, self.velocities = _drift(self.positions, self.velocities, self.charges,
@@ -429,8 +428,9 @@ class ElectrostaticSimulation:
         return tree
 
     def _native_step(self):
-        """The rest of a step after its first fields, the arrays' parts in the library's
-        kernels (one read of the state's facts for the walls and the next fields)."""
+        """A step with the arrays' parts in the library's kernels (one read of the state's
+        facts before the first fields, one for the walls and the next fields)."""
+        self._compute_fields(False, False, self._scan())
         n, stream = self.num_particles, _lib.stream(self.positions.device)
         pos, vel = torch.empty_like(self.positions), torch.empty_like(self.velocities)
         _lib.call("td3_sim_kick_drift", self.positions.data_ptr(), self.velocities.data_ptr(),
@@ -438,9 +438,9 @@ class ElectrostaticSimulation:
                   self.fixed.data_ptr(), n, self.dt, self.B_z, pos.data_ptr(), vel.data_ptr(),
                   stream)
         self.positions, self.velocities = pos, vel
-        facts = self._scan(True)
+        facts = self._scan()
         if self._absorb(facts):
-            facts = self._scan(True)
+            facts = self._scan()
         tree = self._compute_fields(False, False, facts)
         vel, forces = torch.empty_like(self.velocities), torch.empty_like(self.positions)
         _lib.call("td3_sim_kick_force", self.velocities.data_ptr(), self._electric.data_ptr(),
