@@ -441,10 +441,11 @@ int td3_cart_m2l(const int64_t* row_start, const int64_t* partners, int64_t n_ds
                  const double* row_coef, const int* b_start, double* local, void* stream);
 
 /* The mixed-precision td3_cart_m2l for orders up to 16: the same translations in FP32
- * on expansions scaled by the destination cell's half-width (t / h_dst, eps / h_dst,
- * m_a / h_dst^|a|; a source over 64 times larger by its own), the row's sums added to the
- * FP64 locals with h_dst^(-1-|b|) in FP64; dst_half and src_half the cells' half-widths.  Replaces cart_m2l_host (src/tree_d_3d/kernels/
- * cart_m2l_host/cart_m2l_host_pyccel.py:16-80) in the mixed form. */
+ * on expansions scaled by a unit of length u, the power of two nearest the destination cell's
+ * half-width (t / u, eps / u, m_a / u^|a|; from the one nearest the source's where that is more
+ * than 16 times larger), the row's sums added to the FP64 locals with u^(-1-|b|) in FP64;
+ * dst_half and src_half the cells' half-widths.  Replaces cart_m2l_host (src/tree_d_3d/
+ * kernels/cart_m2l_host/cart_m2l_host_pyccel.py:16-80) in the mixed form. */
 int td3_cart_m2l_mixed(const int64_t* row_start, const int64_t* partners, int64_t n_dst,
                        const double* dst_center, const double* dst_half,
                        const double* src_center, const double* src_half,
@@ -454,7 +455,8 @@ int td3_cart_m2l_mixed(const int64_t* row_start, const int64_t* partners, int64_
 /* Source records of td3_cart_m2l_rows, orders up to 16: the bytes of a record (a multiple of
  * 16; TD3_EINVAL for another order), and the records of `count` cells from their Cartesian
  * moments (count, n_coef): (-1)^|a| m_a / (a_x! a_y!) in FP64, or with `mixed` that over
- * h^|a| in FP32, zero beyond the order.  No counterpart in the reference. */
+ * u^|a| in FP32, u the power of two nearest the half-width, zero beyond the order.  No
+ * counterpart in the reference. */
 int td3_cart_record_bytes(int order, int mixed);
 int td3_pack_cart_sources(int64_t count, int order, const double* moments,
                           const double* node_half, int mixed, void* records, void* stream);

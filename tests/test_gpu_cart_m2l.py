@@ -55,6 +55,42 @@ def _oracle_locals(oracle, c, order, start=None, dst_center=None):
     return local
 
 
+@pytest.mark.parametrize("order", [4, 12, 16])
+@pytest.mark.parametrize("packed", [False, True])
+def test_mixed_units_round_nothing(order, packed):
+    """The unit of a cell in the mixed form is a power of two: sizes that change within the same
+    nearest one, in another ratio to each other, give the same bits."""
+    c = _case(order, 1e-3, order)
+    want = _run(c, order, 1, packed)
+    assert np.isfinite(want).all()
+    for scale in (0.93, 1.07):  # 0.1 * 2^k and 1e-3: 1.6 / 16 and 1.024 / 1024, off sqrt(2)
+        other = dict(c, src_half=c["src_half"] * scale, dst_half=c["dst_half"] / scale)
+        assert np.array_equal(_run(other, order, 1, packed), want)
+
+
+@pytest.mark.parametrize("size", [1e-28, 1e30])
+def test_mixed_charges_near_the_ends_of_fp32(oracle, size):
+    """Charges whose moments keep clear of FP32's ends by themselves, but not times the 16th
+    power of the largest ratio of a source's size to its destination's, 16 (tolerances above)."""
+    order, n = 16, 64
+    rng = np.random.default_rng(3)
+    degree = np.array([k for k in range(order + 1) for _ in range(k + 1)])
+    start = np.arange(n + 1, dtype=np.int64)
+    src_half = np.full(n, 0.25)
+    dst_half = 0.25 / 2.0 ** (np.arange(n) % 5)
+    angle = rng.uniform(0, 2 * np.pi, n)
+    c = dict(start=start, partners=np.arange(n, dtype=np.int64), src_half=src_half,
+             dst_half=dst_half, src_center=rng.uniform(-1, 1, (n, 2)),
+             dst_center=5 * np.stack((np.cos(angle), np.sin(angle)), axis=1), degree=degree,
+             moments=size * rng.normal(size=(n, degree.size)) * src_half[:, None] ** degree, eps=0.0)
+    want = _oracle_locals(oracle, c, order)
+    unit = dst_half[:, None] ** degree
+    for packed in (False, True):
+        got = _run(c, order, 1, packed)
+        error = np.max(np.abs(got - want) * unit, axis=1) / np.max(np.abs(want) * unit, axis=1)
+        assert np.all(error < 1e-5)
+
+
 def _off_by_a_double(t):
     """A copy of ``t`` that starts 8 bytes past a 16-byte boundary."""
     copy = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)[1:].view_as(t)

@@ -24,8 +24,8 @@
 // across the row, at whose end the group's 4 lanes are added through shared memory and each
 // lane adds a quarter of the coefficients to the locals: the same bits every run.
 //
-// Mixed precision (T = float): moments in units of the source cell's half-width h_s and
-// sums in units of the destination's h_d; see translate().
+// Mixed precision (T = float): moments in a unit of length near the source cell's half-width,
+// sums in one near the destination's, both powers of two; see unit_of() and translate().
 #include "row_groups.cuh"
 
 #include <type_traits>
@@ -98,6 +98,18 @@ struct Vec<float> {
 struct CartScale {
     double inv_fact2[tri(17)];
 };
+
+// The unit of length of a cell of half-width h in the mixed form: the power of two nearest h,
+// so that every power and ratio of units is exact and a moment is rounded to FP32 once, where
+// it is first an FP32 number, whatever the sizes of the two trees (2^-1000 to 2^1000).
+__device__ __forceinline__ double unit_of(double h) {
+    // the exponent, one higher from a mantissa of sqrt(2) on
+    const int e = (__double2hiint(h) + (0x00100000 - 0x0006a09e)) & 0x7ff00000;
+    return __hiloint2double(min(max(e, 0x01700000), 0x7e700000), 0);
+}
+__device__ __forceinline__ double inverse_unit(double u) {
+    return __hiloint2double(0x7fe00000 - __double2hiint(u), 0);
+}
 
 // 16 bytes to shared memory, zeros without `on` (nothing is then read).
 __device__ __forceinline__ void copy16(unsigned smem, const void* global, bool on) {
@@ -274,11 +286,13 @@ __device__ __forceinline__ void add_translation(const float* part, float* acc) {
     }
 }
 
-// A translation in FP32.  The record's moments are m~_a / h_s^|a| and the sums
-// T~_b h_d^(1+|b|): with t, eps and the moments in units of h_d every product has the sums'
-// unit.  The moments take (h_s / h_d)^|a| here, at most 16^|a|.  A source more than 16 times
-// its destination's size (both units would near the ends of FP32's range) is summed in its
-// own unit h_s and its sums multiplied by (h_d / h_s)^(1+|b|).
+// A translation in FP32, in the units h_s and h_d of source and destination (unit_of).  The
+// record's moments are m~_a / h_s^|a| and the sums T~_b h_d^(1+|b|): with t, eps and the moments
+// in units of h_d every product has the sums' unit.  The moments take (h_s / h_d)^|a| here, at
+// most 16^|a|; where that grows, half of the highest power goes to A~ instead (a charge of 1e30
+// times 16^16 is beyond FP32).  A source more than 16 times its destination's size (both units
+// would near the ends of FP32's range) is summed in its own unit h_s and its sums multiplied by
+// (h_d / h_s)^(1+|b|).
 constexpr double UNIT_RANGE = 16.0;
 
 template <int P, int B0, int B1>
@@ -286,15 +300,24 @@ __device__ __forceinline__ void translate(float* m, double tx, double ty, double
                                           double hd, int order, float* acc) {
     constexpr int NA = P - B0, NB = Products<float, P, B0, B1>::NB;
     const bool far_unit = hs > UNIT_RANGE * hd;
-    const double inv = 1.0 / (far_unit ? hs : hd);
+    const double inv = inverse_unit(far_unit ? hs : hd);
     const float x = (float)(tx * inv), y = (float)(ty * inv);
     const float r2 = (float)((double)x * x + (double)y * y + eps2 * inv * inv);
-    const float a0 = rsqrtf(r2), ir2 = 1.0f / r2;
+    const float ir2 = 1.0f / r2;
+    float a0 = rsqrtf(r2);
     if (!far_unit) {
         if (hs != hd) {
             const float f = (float)(hs * inv);
             float p[NA + 1];
             p[0] = 1.0f;
+            if (f > 1.0f) {
+                const float g = 1.0f / f;
+#pragma unroll
+                for (int k = 0; k < NA / 2; ++k) {
+                    p[0] *= g;
+                    a0 *= f;
+                }
+            }
 #pragma unroll
             for (int k = 1; k <= NA; ++k) p[k] = p[k - 1] * f;
             static_for<words_of(tri(NA + 1), 4)>([&](auto wc) {
@@ -363,8 +386,8 @@ k_m2l_cart_rows(const i64* __restrict__ row_start, const i64* __restrict__ partn
             tx = dst_center[2 * d] - src_center[2 * (i64)src];
             ty = dst_center[2 * d + 1] - src_center[2 * (i64)src + 1];
             if (MIXED) {
-                hs = src_half[src];
-                hd = dst_half[d];
+                hs = unit_of(src_half[src]);
+                hd = unit_of(dst_half[d]);
             }
         }
         __syncwarp();
@@ -390,7 +413,7 @@ k_m2l_cart_rows(const i64* __restrict__ row_start, const i64* __restrict__ partn
             for (int p = 0; p < 32; ++p) {
                 const int s = __shfl_sync(FULL_WARP, src, p);
                 if (s < 0) continue;
-                const double inv_h = MIXED ? 1.0 / src_half[s] : 1.0;
+                const double inv_h = MIXED ? inverse_unit(unit_of(src_half[s])) : 1.0;
                 // zeros above the order, as in a record: products() multiplies degree order + 1
                 // by 0, and what shared memory held may be a NaN
                 for (int a = lane; a < tri(NA + 1); a += 32) {
@@ -431,7 +454,7 @@ k_m2l_cart_rows(const i64* __restrict__ row_start, const i64* __restrict__ partn
         for (int k = 0; k < Q; ++k) was[k] = k < count ? out[k] : 0.0;
         double unit = 1.0;
         int n = -1;  // the degree that `unit` = h_d^-(1 + n) belongs to
-        const double inv_h = MIXED ? 1.0 / dst_half[d] : 1.0;
+        const double inv_h = MIXED ? inverse_unit(unit_of(dst_half[d])) : 1.0;
 #pragma unroll
         for (int k = 0; k < Q; ++k) {
             if (k < count) {
@@ -476,7 +499,7 @@ k_m2l_cart_rows(const i64* __restrict__ row_start, const i64* __restrict__ partn
         });
 }
 
-// Records for the M2L: m~_a (FP64), or m~_a / h^|a| (FP32); zero beyond the order.
+// Records for the M2L: m~_a (FP64), or m~_a / unit^|a| (FP32); zero beyond the order.
 template <typename T, int P>
 __global__ void k_pack_cart(i64 count, int order, const double* __restrict__ moments,
                             const double* __restrict__ half, const CartScale C,
@@ -495,7 +518,7 @@ __global__ void k_pack_cart(i64 count, int order, const double* __restrict__ mom
             v = moments[node * n_coef + a] * C.inv_fact2[a];
             if (na & 1) v = -v;
             if (sizeof(T) == 4) {
-                const double inv_h = 1.0 / half[node];
+                const double inv_h = inverse_unit(unit_of(half[node]));
                 for (int k = 0; k < na; ++k) v *= inv_h;
             }
         }
