@@ -55,6 +55,13 @@ def _oracle_locals(oracle, c, order, start=None, dst_center=None):
     return local
 
 
+@pytest.mark.parametrize("order", range(17))
+@pytest.mark.parametrize("mixed", [0, 1])
+def test_plain_moments_are_scaled_to_the_bits_of_records(order, mixed):
+    c = _case(order, 1e-3, 50 + order)
+    assert np.array_equal(_run(c, order, mixed, False), _run(c, order, mixed, True))
+
+
 @pytest.mark.parametrize("order", [4, 12, 16])
 @pytest.mark.parametrize("packed", [False, True])
 def test_mixed_units_round_nothing(order, packed):

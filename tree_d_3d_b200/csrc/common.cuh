@@ -186,7 +186,7 @@ int td3_m2l_log_rows(const i64* row_start, const i64* partners, i64 n_dst,
                      const double* moment_im, int order, const double* coeff, double* local_re,
                      double* local_im, cudaStream_t s);
 
-// The Cartesian M2L of orders up to 16 from the moments themselves (cart_m2l.cu): arguments
+// The Cartesian M2L of orders up to 16 from the moments themselves (cart_m2l_plain.cu): arguments
 // as td3_cart_m2l_mixed; FP64 without `mixed` (the half-widths are then not read).
 int td3_cart_m2l_unpacked(const i64* row_start, const i64* partners, i64 n_dst,
                           const double* dst_center, const double* dst_half,

@@ -3,7 +3,7 @@
 //   L2L per level           (K/cart_downward/cart_downward_pyccel.py:14-55)
 // (moments: moments.cu; L2P + P2P: nearfield.cu.)
 //
-// M2L (orders above 16; up to 16: cart_m2l.cu): one warp per destination cell.  For each
+// M2L (orders above 16; up to 16: cart_m2l.cuh): one warp per destination cell.  For each
 // partner the warp builds the Taylor coefficients A_g(t), |g| <= p, of f = (|r|^2 + eps^2)^(-1/2) degree by degree in
 // shared memory (the coefficients of one degree depend only on the two below), then
 // every lane accumulates its local coefficients b over the M2L rows (b, a, a + b) of

@@ -1,4 +1,4 @@
-// The walk of a warp over CSR rows of an M2L with a lane per entry (cart_m2l.cu,
+// The walk of a warp over CSR rows of an M2L with a lane per entry (cart_m2l.cuh,
 // m2l_log_rows.cu): groups of ROW_GL lanes take the warp's rows in order, lane i of a group
 // the entries i, i + ROW_GL, ... of its row; rows above LONG_ROW entries are taken by the
 // whole warp first.  Each row is summed by one group or warp in a fixed order.
