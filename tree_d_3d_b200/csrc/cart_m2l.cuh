@@ -231,7 +231,9 @@ struct Products {
                 products<n, true, true>(m, e, o, order, acc);
             } else {
                 products<n, true, false>(m, e, o, order, acc);
-                if constexpr (n + 1 <= P) products<n, false, true>(m, e, o, order, acc);
+                if constexpr (n + 1 <= P) {
+                    if (n + 1 <= order) products<n, false, true>(m, e, o, order, acc);
+                }
             }
             step<n + 2>(m, e, o, tx, ty, ir2, order, acc);
         }
