@@ -132,7 +132,7 @@ def _run(c, order, mixed, packed, shift=False):
 
 
 @pytest.mark.parametrize("order,eps", [(1, 0.0), (4, 1e-3), (5, 0.5), (8, 0.0), (11, 1e-3),
-                                       (12, 0.5), (14, 0.0), (16, 1e-3)])
+                                       (12, 0.5), (13, 0.5), (14, 0.0), (16, 1e-3)])
 def test_cartesian_m2l_rows_match_the_oracle(oracle, order, eps):
     c = _case(order, eps, 100 + order)
     want = _oracle_locals(oracle, c, order)

@@ -44,10 +44,11 @@ int launch_pack(i64 count, int order, const double* moments, const double* half,
 
 extern "C" int td3_cart_record_bytes(int order, int mixed) {
     if (order < 0 || order > 16) return TD3_EINVAL;
-    switch (template_order(order)) {
+    switch (template_order(order, mixed != 0)) {
         case 4: return 16 * (mixed ? WORDS<float, 4> : WORDS<double, 4>);
         case 8: return 16 * (mixed ? WORDS<float, 8> : WORDS<double, 8>);
         case 12: return 16 * (mixed ? WORDS<float, 12> : WORDS<double, 12>);
+        case 14: return 16 * WORDS<double, 14>;
         default: return 16 * (mixed ? WORDS<float, 16> : WORDS<double, 16>);
     }
 }
@@ -58,7 +59,7 @@ extern "C" int td3_pack_cart_sources(int64_t count, int order, const double* mom
     if (count < 0 || order < 0 || order > 16) return TD3_EINVAL;
     if (count == 0) return TD3_OK;
     cudaStream_t s = td3_stream(stream);
-    switch (template_order(order)) {
+    switch (template_order(order, mixed != 0)) {
         case 4:
             return mixed ? launch_pack<float, 4>(count, order, moments, node_half, records, s)
                          : launch_pack<double, 4>(count, order, moments, node_half, records, s);
@@ -68,6 +69,7 @@ extern "C" int td3_pack_cart_sources(int64_t count, int order, const double* mom
         case 12:
             return mixed ? launch_pack<float, 12>(count, order, moments, node_half, records, s)
                          : launch_pack<double, 12>(count, order, moments, node_half, records, s);
+        case 14: return launch_pack<double, 14>(count, order, moments, node_half, records, s);
         default:
             return mixed ? launch_pack<float, 16>(count, order, moments, node_half, records, s)
                          : launch_pack<double, 16>(count, order, moments, node_half, records, s);
