@@ -60,7 +60,9 @@ const char* td3_last_error(void);
  * (phi = sum q / sqrt(r^2 + eps^2)) or TD3_KERNEL_LOG (phi = -sum q ln(r^2 + eps^2),
  * E = 2 sum q d / (r^2 + eps^2)).  exclude[i] is a source index skipped for target i
  * (-1: none); zero charges are skipped.  with_potential = 0 writes phi = 0 and, for
- * the log kernel, skips the logarithms.
+ * the log kernel, skips the logarithms.  The sources are summed in chunks whose partial sums
+ * the workspace holds; one shorter than its query takes fewer chunks, down to 24 n_targets
+ * bytes per 2048 sources (none for up to 2048), below which the call is refused.
  * Replaces the reference kernels direct_sum (src/tree_d_3d/kernels/direct_sum/
  * direct_sum_cuda.cu:7-44) and direct_log_sum (kernels/direct_log_sum/
  * direct_log_sum_cuda.cu:7-42), called by direct_field (src/tree_d_3d/flat_tree.py:157-158). */
@@ -79,9 +81,9 @@ int td3_direct_sum(int kernel, const double* targets, int64_t n_targets, const i
  * The first call on a device looks up the array's device address (once per device,
  * with that device current); make that first call before any stream capture.  The
  * address stays cached until the process exits: do not reset a device
- * (cudaDeviceReset) between calls of this entry point.  Every call shares the array:
- * calls that overlap on the GPU (other streams, other threads) race on it, so
- * serialise them.  Results equal td3_direct_sum's. */
+ * (cudaDeviceReset) between calls of this entry point.  Every call of more than 2048 sources
+ * shares the array: calls that overlap on the GPU (other streams, other threads) race on it,
+ * so serialise them.  Results equal td3_direct_sum's but for the order of the chunks' sums. */
 #define TD3_DIRECT_NOALLOC_MAX_TARGETS 65536
 int td3_direct_sum_noalloc(int kernel, const double* targets, int64_t n_targets,
                            const int64_t* exclude, const double* pos, const double* charge,

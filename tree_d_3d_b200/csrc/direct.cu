@@ -125,11 +125,13 @@ __global__ void k_direct_reduce(const double* __restrict__ partial, i64 m, int c
 
 // Source chunks so that (target blocks x chunks) fills the GPU a few times over, with at
 // least 64 sources per chunk: 1000 targets of 1000 sources take 16 chunks (one block per 256
-// targets and all sources ran 0.12 ms on 4 SMs).
-int direct_chunks(i64 m, i64 n) {
+// targets and all sources ran 0.12 ms on 4 SMs).  Without scratch of its caller's a call takes
+// chunks of LONG_CHUNK at least, which no call of up to as many sources needs scratch for.
+constexpr i64 CHUNK = 64, LONG_CHUNK = 2048;
+int direct_chunks(i64 m, i64 n, i64 least) {
     i64 bx = (m + DIRECT_THREADS - 1) / DIRECT_THREADS;
     i64 want = (4 * SM_COUNT_B200 + bx - 1) / bx;
-    i64 most = (n + 63) / 64;
+    i64 most = (n + least - 1) / least;
     i64 c = want < most ? want : most;
     if (c > 256) c = 256;
     return (int)(c < 1 ? 1 : c);
@@ -217,7 +219,7 @@ __global__ void k_sum_into(const double* __restrict__ partial, i64 count, double
 }  // namespace
 
 extern "C" size_t td3_direct_sum_workspace_size(int64_t n_targets, int64_t n_sources) {
-    int chunks = direct_chunks(n_targets, n_sources);
+    int chunks = direct_chunks(n_targets, n_sources, CHUNK);
     return chunks > 1 ? td3_ws_bytes<double>(3 * (i64)chunks * n_targets) : 256;
 }
 
@@ -235,9 +237,15 @@ extern "C" int td3_direct_sum(int kernel, const double* targets, int64_t m, cons
         TD3_TRY(cudaMemsetAsync(field, 0, sizeof(double) * 2 * m, s));
         return TD3_OK;
     }
-    int chunks = direct_chunks(m, n);
-    if (chunks > 1 && workspace_bytes < (size_t)3 * chunks * m * sizeof(double))
-        return TD3_EWORKSPACE;
+    // as many chunks as the workspace holds, LONG_CHUNK's at least
+    int chunks = direct_chunks(m, n, CHUNK);
+    const size_t per_chunk = (size_t)3 * m * sizeof(double);
+    if (chunks > 1 && workspace_bytes / per_chunk < (size_t)chunks) {
+        const int least = direct_chunks(m, n, LONG_CHUNK);
+        chunks = (int)(workspace_bytes / per_chunk);
+        if (chunks < 1) chunks = 1;
+        if (chunks < least) return TD3_EWORKSPACE;
+    }
     double* partial = static_cast<double*>(workspace);
     double eps2 = softening * softening;
     bool pot = with_potential != 0;
@@ -282,8 +290,8 @@ extern "C" int td3_pair_energy(const double* pos, const double* charge, int64_t 
 // the source chunks -- lives in the array below, a fixed part of every device that
 // loads the library, kept until the process exits.  The array holds the partial sums
 // of any call with at most TD3_DIRECT_NOALLOC_MAX_TARGETS targets (any number of
-// sources): 3 x chunks x targets doubles, at most 605,184 (4.6 MiB) for the chunk
-// counts that td3_direct_sum chooses.
+// sources): 3 x chunks x targets doubles, at most 605,184 (4.6 MiB) for chunks of LONG_CHUNK
+// sources; calls of up to LONG_CHUNK sources leave it alone.
 namespace {
 
 constexpr i64 NOALLOC_SCRATCH_DOUBLES = 605184;
@@ -338,7 +346,7 @@ extern "C" int td3_direct_sum_noalloc(int kernel, const double* targets, int64_t
         TD3_TRY(cudaMemsetAsync(field, 0, sizeof(double) * 2 * m, s));
         return TD3_OK;
     }
-    int chunks = direct_chunks(m, n);
+    int chunks = direct_chunks(m, n, LONG_CHUNK);
     if (chunks > 1 && (i64)3 * chunks * m > NOALLOC_SCRATCH_DOUBLES) {
         td3_set_error("td3_direct_sum_noalloc: the partial sums exceed the fixed scratch");
         return TD3_ETOOLARGE;
