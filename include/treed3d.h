@@ -21,7 +21,8 @@
  * Entry points are re-entrant and keep no state between calls, with one exception:
  * td3_direct_sum_noalloc keeps its scratch in one fixed device array shared by all of
  * its calls (and caches that array's address per device), so its calls must not
- * overlap on the GPU; its block below gives the details.
+ * overlap on the GPU; its block below gives the details.  (Some entry points also look up
+ * once per device how many blocks of a kernel it holds.)
  */
 #ifndef TREED3D_H
 #define TREED3D_H

@@ -35,8 +35,6 @@
 
 namespace {
 
-constexpr int MAX_DEVICES = 64;
-
 __host__ __device__ constexpr int tri(int n) { return n * (n + 1) / 2; }
 __host__ __device__ constexpr double factorial(int n) { return n < 2 ? 1.0 : n * factorial(n - 1); }
 __host__ __device__ constexpr int degree_of(int i) {
@@ -580,11 +578,10 @@ int launch_rows(const Args& a) {
     auto kernel = k_m2l_cart_rows<T, P, B0, B1, PLAIN>;
     constexpr size_t smem = sizeof(T) * 32 * STAGE_PITCH<T, P, B0, B1, PLAIN> * WARPS_PER_BLOCK<T>;
     // one resident wave of blocks, each warp an even share of the entries
-    // (the per-device figures are cached; concurrent first calls store the same values)
-    static int blocks_of[MAX_DEVICES] = {};
+    static td3_per_device blocks_of;
     int dev = 0;
     TD3_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= MAX_DEVICES) return TD3_EINVAL;
+    if (dev < 0 || dev >= TD3_MAX_DEVICES) return TD3_EINVAL;
     if (!blocks_of[dev]) {
         int sms = 0, per_sm = 0;
         TD3_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "treed3d.h"
 
 typedef int64_t i64;
@@ -163,6 +165,11 @@ struct td3_i64x2 {
 };
 
 // ---------------------------------------------------------------------------------
+// Per-device block counts that a launch function looks up once: the only state that calls share,
+// read and written as atomics (concurrent first calls store the same values).
+constexpr int TD3_MAX_DEVICES = 64;
+typedef std::atomic<int> td3_per_device[TD3_MAX_DEVICES];
+
 // Device-wide scans (scan.cu).  Exclusive scan of n items; total (optional) receives the sum.
 size_t td3_scan_workspace(i64 n);
 int td3_exclusive_scan_i64(const i64* in, i64* out, i64 n, i64* total, void* ws, size_t ws_bytes,

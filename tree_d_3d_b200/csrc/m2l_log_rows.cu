@@ -15,8 +15,6 @@
 
 namespace {
 
-constexpr int MAX_DEVICES = 64;
-
 // 8 bytes to shared memory, zero without `on` (nothing is then read).
 __device__ __forceinline__ void copy8(unsigned smem, const double* global, bool on) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem), "l"(global),
@@ -172,11 +170,10 @@ int launch_rows(const i64* row_start, const i64* partners, i64 n_dst, const doub
                 const double* coeff, double* lre, double* lim, cudaStream_t s) {
     auto kernel = k_m2l_log_rows<P>;
     // one resident wave of one-warp blocks, each an even share of the entries
-    // (the per-device figures are cached; concurrent first calls store the same values)
-    static int blocks_of[MAX_DEVICES] = {};
+    static td3_per_device blocks_of;
     int dev = 0;
     TD3_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= MAX_DEVICES) return TD3_EINVAL;
+    if (dev < 0 || dev >= TD3_MAX_DEVICES) return TD3_EINVAL;
     if (!blocks_of[dev]) {
         int sms = 0, per_sm = 0;
         TD3_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,

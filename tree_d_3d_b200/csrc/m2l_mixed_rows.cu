@@ -25,7 +25,6 @@ constexpr int GL = 8;          // lanes per destination group
 constexpr int LONG_ROW = 96;   // rows longer than this are taken by the whole warp
 constexpr int ROW_COST = GL;   // entries a row counts for in the warps' shares
 constexpr unsigned FULL = 0xffffffffu;
-constexpr int MAX_DEVICES = 64;
 
 template <int P>
 struct RowCoef {
@@ -319,20 +318,17 @@ int launch_rows(const i64* row_start, const i64* partners, i64 n_dst, const doub
         for (int l = 0; l <= P; ++l)
             C.c[k * (P + 1) + l] = (k < w && l < w) ? (float)coeff[k * w + l] : 0.0f;
     // one resident wave of blocks, each warp an even share of the entries
-    // (the per-device figures are cached; concurrent first calls store the same values)
-    static int per_sm[MAX_DEVICES] = {};
-    static int sms[MAX_DEVICES] = {};
+    static td3_per_device blocks_of;
     int dev = 0;
     TD3_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= MAX_DEVICES) return TD3_EINVAL;
-    if (!per_sm[dev]) {
+    if (dev < 0 || dev >= TD3_MAX_DEVICES) return TD3_EINVAL;
+    if (!blocks_of[dev]) {
         int n = 0, b = 0;
         TD3_TRY(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
         TD3_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_m2l_mixed_rows<P>, 32 * RW, 0));
-        sms[dev] = n;
-        per_sm[dev] = b > 0 ? b : 1;
+        blocks_of[dev] = n * (b > 0 ? b : 1);
     }
-    i64 blocks = (i64)sms[dev] * per_sm[dev];
+    i64 blocks = blocks_of[dev];
     const i64 max_blocks = (n_dst + RW - 1) / RW;
     if (blocks > max_blocks) blocks = max_blocks;
     TD3_TRY(td3_launch_chained(k_m2l_mixed_rows<P>, (unsigned)blocks, 32 * RW, 0, s, row_start,
