@@ -182,7 +182,8 @@ int launch_rows(const i64* row_start, const i64* partners, i64 n_dst, const doub
         TD3_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32, 0));
         blocks_of[dev] = sms * (per_sm > 0 ? per_sm : 1);
     }
-    const i64 blocks = n_dst < blocks_of[dev] ? n_dst : blocks_of[dev];
+    i64 blocks = blocks_of[dev];
+    if (blocks > n_dst) blocks = n_dst;
     TD3_TRY(td3_launch_chained(kernel, (unsigned)blocks, 32, 0, s, row_start, partners, n_dst,
                                dst_center, src_center, mre, mim, order, coeff, lre, lim));
     return TD3_OK;
