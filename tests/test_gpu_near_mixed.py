@@ -29,16 +29,22 @@ def _run(pos, q, kernel, eps, precision, split, w, e, overlap=True):
     return [t.detach().cpu().numpy() for t in (phi, field, Q.grad, P.grad)]
 
 
-@pytest.mark.parametrize("segment", [256, 8])
+@pytest.mark.parametrize("segment", [256, 64, 8])
 @pytest.mark.parametrize("kernel,eps", [("log", 0.0), ("log", 1e-3), ("coulomb", 1e-3)])
 def test_split_near_field_matches_one_launch_form_and_fp64(kernel, eps, segment, monkeypatch):
     from tree_d_3d_b200 import flat_tree, synthetic
 
-    # segment 8: most leaves take several segments (the partial-sum path)
-    monkeypatch.setattr(flat_tree, "NEAR_SEGMENT", segment)
+    # 64 is the package's own; 8: most leaves take several segments (the partial-sum path)
+    if segment != 64:
+        monkeypatch.setattr(flat_tree, "NEAR_SEGMENT", segment)
+        monkeypatch.setattr(flat_tree, "NEAR_SEGMENT_PARTICLES", 8 * segment)
     monkeypatch.setattr(flat_tree, "NEAR_SPLIT", True)
     monkeypatch.setattr(flat_tree, "NEAR_OVERLAP", True)
     pos, q = synthetic.mixture8(60_000, seed=70)
+    lists = flat_tree.FlatQuadtree(pos, q, flat_tree.Quad(0, 0, 1), kernel="log")._lists(0.5)
+    rows, plan = lists["p2p_rows"], lists["plan"]
+    parts = plan["seg_range"][: plan["n_seg"]]
+    assert int((parts[:, 1] - parts[:, 0]).max()) == min(segment, int((rows[1:] - rows[:-1]).max()))
     rng = np.random.default_rng(71)
     w = torch.tensor(rng.normal(size=pos.shape[1]), device="cuda")
     e = torch.tensor(rng.normal(size=pos.shape), device="cuda")

@@ -484,9 +484,9 @@ int launch_log_moments(const int64_t* levels, int64_t n_levels, int order, const
             if (hi <= lo) continue;
             const size_t smem = sizeof(double2) * LOG_MOM_WARPS * LOG_MOM_SLOTS * (sdip ? 2 : 1) *
                                 ((order + 1) | 1);
-            if (smem > 48 * 1024)
-                TD3_TRY(cudaFuncSetAttribute(k_log_moments, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem));
+            static_assert(sizeof(double2) * LOG_MOM_WARPS * LOG_MOM_SLOTS * 2 *
+                                  ((TD3_MAX_ORDER + 1) | 1) <= 48 * 1024,
+                          "k_log_moments asks for no more shared memory than every launch may");
             TD3_TRY(td3_launch_chained(k_log_moments,
                                        (unsigned)((hi - lo + LOG_MOM_WARPS - 1) / LOG_MOM_WARPS),
                                        32 * LOG_MOM_WARPS, smem, s, lo, hi, order, spos, scharge, n,

@@ -15,6 +15,8 @@
 
 constexpr int ROW_GL = 4;                // lanes per row
 constexpr int ROW_GROUPS = 32 / ROW_GL;  // rows in flight per warp
+constexpr unsigned ROW_LEADERS = 0xffffffffu / ((1u << ROW_GL) - 1u);  // each group's lane 0
+static_assert(ROW_GL == 4 && ROW_LEADERS == 0x11111111u, "the row sums add four lanes by name");
 constexpr int LONG_ROW = 256;            // rows longer than this are taken by the whole warp,
 constexpr int FEW_ROWS = 6;              // or, with at most so many rows per warp,
 constexpr int LONG_OF_FEW = 8;           // rows longer than this
@@ -106,7 +108,7 @@ __device__ __forceinline__ void walk_rows(const i64* __restrict__ row_start,
                 to = whole ? claim(row, true) : claim(da + g, false);
             } else {
                 // the finished groups take the next rows, in group order
-                const unsigned gm = dm & 0x11111111u;
+                const unsigned gm = dm & ROW_LEADERS;
                 if (done) to = claim(next + __popc(gm & ((1u << (ROW_GL * g)) - 1u)), false);
                 next += __popc(gm);
             }
