@@ -135,6 +135,23 @@ def test_fmm_at_matches_oracle_on_large_targets(oracle, kernel):
     assert relative(_np(b[1]), a[1]) < TOL
 
 
+@pytest.mark.parametrize("kernel", ["log", "coulomb"])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("count,spread", [(1, 0.0), (40, 0.0), (2, 1e-15), (30, 1e-12)])
+def test_fmm_at_one_point(kernel, precision, count, spread):
+    """One target, the same one many times and targets next to each other against the direct
+    sum: the truncation of order 12 at theta 0.5 is below 1e-4 of either."""
+    from tree_d_3d_b200 import FlatQuadtree, Quad, direct_field, synthetic
+
+    pos, q = synthetic.mixture8(2000, seed=3)
+    targets = np.full((2, count), 0.85) + spread * np.arange(count) / max(count - 1, 1)
+    tree = FlatQuadtree(pos, q, Quad(0, 0, 1), kernel=kernel, order=12, precision=precision)
+    got = tree.fmm_at(targets, softening=1e-3)
+    want = direct_field(targets, pos, q, softening=1e-3, kernel=kernel)
+    for a, b in zip(got, want):
+        assert relative(a, b) < 1e-4
+
+
 def test_fmm_at_keeps_its_plan_across_new_charges():
     from tree_d_3d_b200 import FlatQuadtree, Quad
 

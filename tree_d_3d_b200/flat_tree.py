@@ -1195,6 +1195,9 @@ class FlatQuadtree:
         hi = targets.amax(dim=1).tolist()
         centre = (0.5 * (lo[0] + hi[0]), 0.5 * (lo[1] + hi[1]))
         half = 0.5 * max(hi[0] - lo[0], hi[1] - lo[1]) * (1 + 1e-12) + 1e-300
+        # one point, or the same one again: a cell that the mixed M2L can take for its unit of
+        # length (its powers overflow with 1e-300)
+        half = max(half, 2.0 ** -40 * self.root_quad.half)
         tree = FlatQuadtree(targets, torch.zeros(m, dtype=torch.float64, device=self.device),
                             Quad(centre[0], centre[1], half), leaf_capacity=leaf,
                             max_depth=self.max_depth, kernel="coulomb")
