@@ -487,7 +487,7 @@ int td3_cart_downward(const int64_t* levels, int64_t n_levels, const double* nod
 
 /* The work plan of the near field: every non-empty leaf's row of P2P partners
  * (rows: n_nodes + 1 offsets, td3_pair_csr) cut into segments of at most `segment`
- * partners.  seg_leaf (int32), seg_range (e0, e1 pairs) and seg_out (-1: the leaf has
+ * partners, or a 256th of the row where that is more.  seg_leaf (int32), seg_range (e0, e1 pairs) and seg_out (-1: the leaf has
  * one segment and writes its final values; else the offset, in targets, of the
  * segment's partial sums) receive n_seg entries; sizes (HOST, 2) = n_seg and the
  * partial length (the caller allocates 3 * partial length doubles for the evaluation).

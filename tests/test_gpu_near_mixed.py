@@ -44,7 +44,8 @@ def test_split_near_field_matches_one_launch_form_and_fp64(kernel, eps, segment,
     lists = flat_tree.FlatQuadtree(pos, q, flat_tree.Quad(0, 0, 1), kernel="log")._lists(0.5)
     rows, plan = lists["p2p_rows"], lists["plan"]
     parts = plan["seg_range"][: plan["n_seg"]]
-    assert int((parts[:, 1] - parts[:, 0]).max()) == min(segment, int((rows[1:] - rows[:-1]).max()))
+    longest = int((rows[1:] - rows[:-1]).max())
+    assert int((parts[:, 1] - parts[:, 0]).max()) == min(max(segment, -(-longest // 256)), longest)
     rng = np.random.default_rng(71)
     w = torch.tensor(rng.normal(size=pos.shape[1]), device="cuda")
     e = torch.tensor(rng.normal(size=pos.shape), device="cuda")
@@ -59,6 +60,40 @@ def test_split_near_field_matches_one_launch_form_and_fp64(kernel, eps, segment,
         assert np.array_equal(a, s1)
         assert relative(a, c) < 1e-6
         assert relative(a, d) < 1e-6
+
+
+@pytest.mark.parametrize("length", [0, 1, 63, 64, 65, 16384, 16385, 16640, 16641, 70_001])
+@pytest.mark.parametrize("segment", [64, 16])
+def test_plan_of_long_rows(length, segment):
+    """A leaf's row cut by `segment` partners, or into 256 where that is fewer parts: the parts
+    follow each other, and their partial sums have room."""
+    from tree_d_3d_b200 import _lib
+
+    dev = torch.device("cuda")
+    rows = torch.tensor([0, 5, 5 + length, 10 + length], device=dev)  # three leaves
+    child = torch.full((3,), -1, dtype=torch.int64, device=dev)
+    start = torch.tensor([0, 2, 9], device=dev)
+    end = torch.tensor([2, 9, 12], device=dev)
+    capacity = 3 + (10 + length) // segment + 1
+    leaf = torch.zeros(capacity, dtype=torch.int32, device=dev)
+    parts = torch.zeros((capacity, 2), dtype=torch.int64, device=dev)
+    at = torch.zeros(capacity, dtype=torch.int64, device=dev)
+    sizes = np.zeros(2, dtype=np.int64)
+    ws = _lib.workspace(_lib.query("td3_nearfield_plan_workspace_size", 3), dev)
+    _lib.call("td3_nearfield_plan", rows.data_ptr(), 3, child.data_ptr(), start.data_ptr(),
+              end.data_ptr(), segment, leaf.data_ptr(), parts.data_ptr(), at.data_ptr(), capacity,
+              sizes.ctypes.data, ws.data_ptr(), ws.numel(), _lib.stream())
+    part = max(segment, -(-length // 256))
+    cuts = list(range(5, 5 + length, part)) or [5]
+    want = [(0, 0, 5, -1)]
+    want += [(1, c, min(c + part, 5 + length), 7 * k if len(cuts) > 1 else -1)
+             for k, c in enumerate(cuts)]
+    want += [(2, 5 + length, 10 + length, -1)]
+    n = int(sizes[0])
+    got = [(int(a), int(b[0]), int(b[1]), int(c)) for a, b, c in
+           zip(leaf[:n].tolist(), parts[:n].tolist(), at[:n].tolist())]
+    assert got == want
+    assert sizes[1] == (7 * len(cuts) if len(cuts) > 1 else 0)
 
 
 def test_split_near_field_reports_coincident_charges(monkeypatch):

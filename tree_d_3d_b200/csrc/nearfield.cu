@@ -38,6 +38,16 @@ __device__ __forceinline__ int pow2_at_least(int v) {
 }
 
 // ------------------------------------------------------------------ the plan
+// Partners per segment of a row of `len`: `segment`, but a row is cut into MAX_SEGMENTS at the
+// most.  One warp adds the segments' sums, in order: a row of 72,736 partners (1M clustered
+// particles) cut by 64 took it 0.27 ms in the mixed field and 0.22 in its backward, by a 256th
+// of the row 0.07 and 0.06 ms.
+constexpr i64 MAX_SEGMENTS = 256;
+__device__ __forceinline__ i64 row_segment(i64 len, int segment) {
+    const i64 least = (len + MAX_SEGMENTS - 1) / MAX_SEGMENTS;
+    return least > segment ? least : segment;
+}
+
 __global__ void k_plan_count(i64 n_nodes, const i64* __restrict__ rows, const i64* __restrict__ child,
                              const i64* __restrict__ start, const i64* __restrict__ end, int segment,
                              i64* __restrict__ nseg, i64* __restrict__ psize) {
@@ -49,7 +59,8 @@ __global__ void k_plan_count(i64 n_nodes, const i64* __restrict__ rows, const i6
     i64 s = 0;
     if (child[n] < 0 && count > 0) {
         i64 len = rows[n + 1] - rows[n];
-        s = len <= segment ? 1 : (len + segment - 1) / segment;
+        const i64 part = row_segment(len, segment);
+        s = len <= part ? 1 : (len + part - 1) / part;
     }
     nseg[n] = s;
     psize[n] = s > 1 ? s * count : 0;
@@ -68,9 +79,10 @@ __global__ void k_plan_fill(i64 n_nodes, const i64* __restrict__ rows, const i64
     if (s == 0) return;
     i64 first = nseg_scan[n], count = end[n] - start[n];
     i64 r0 = rows[n], r1 = rows[n + 1];
+    const i64 part = row_segment(r1 - r0, segment);
     for (i64 k = 0; k < s; ++k) {
-        i64 e0 = r0 + k * segment;
-        i64 e1 = e0 + segment < r1 ? e0 + segment : r1;
+        i64 e0 = r0 + k * part;
+        i64 e1 = e0 + part < r1 ? e0 + part : r1;
         if (s == 1) e1 = r1;
         seg_leaf[first + k] = (int)n;
         seg_range[first + k] = make_longlong2(e0, e1);

@@ -181,7 +181,8 @@ def _m2l_coefficients(order: int, symmetric: bool) -> np.ndarray:
 #: particles a segment may hold: the launch ends with its longest segment (a warp's 256
 #: partners of 16 particles took 0.2 ms alone).  48k panel nodes: 1.16 -> 0.90 ms per product
 #: with 64 partners instead of 256; 50k strip charges (leaves of 32): 2.9 -> 2.6 ms with 32.
-#: Shorter ones cost the 1M-particle fields more partial sums (2 to 4 % at 16 partners).
+#: Shorter ones cost the 1M-particle fields more partial sums (2 to 4 % at 16 partners).  The
+#: plan cuts no row into more than 256.
 NEAR_SEGMENT = 64
 NEAR_SEGMENT_PARTICLES = 1024
 
