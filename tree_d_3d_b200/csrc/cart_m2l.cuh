@@ -15,10 +15,9 @@
 // products per value read (with A and the moments both there the reads cost twice the
 // products' time).
 //
-// Measured (1M clustered particles, theta 0.5, 12.6M translations, records included): p = 12
-// FP64 18.6 -> 5.6 ms against a lane per coefficient run with both
-// operands in shared memory, FP32 4.5 ms (100k particles, two launches of the backward
-// step: 2.3 -> 0.9 ms).
+// Measured (1M clustered particles, theta 0.5, 12.6M translations, records included; a lane per
+// coefficient run with both operands in shared memory before): p = 12 FP64 18.6 -> 5.6 ms, FP32
+// 13.2 -> 4.5 ms (100k particles, the two of a backward step: 2.3 -> 0.9 ms).
 //
 // Work: a warp walks its rows with four lanes per row (walk_rows); a lane keeps its sums
 // across the row, at whose end the group's 4 lanes are added through shared memory and each
